@@ -178,6 +178,88 @@ def run(s):
     return s["dq"], s["dkv"], delta[:, :, :s["sq"]]
 
 
+def _visible(case, s0, s1, q_off, sk):
+    """Which of keys 0..sk-1 queries s0..s1-1 see: (number of leading keys that matter, mask of those or None)."""
+    if not case["causal"]:
+        return sk, None
+    n = min(max(q_off + s1, 0), sk)
+    pos = torch.arange(s0, s1, device="cuda")[:, None] + q_off
+    return n, torch.arange(n, device="cuda")[None, :] > pos
+
+
+def _exact_forward(case, q, k, v, q_off, chunk=2048):
+    """o [B,S,H,D] and lse [B,H,S] of plain attention in fp64."""
+    b, sq, hq, d = q.shape
+    sk, group = k.shape[1], hq // k.shape[2]
+    o = torch.zeros(b, sq, hq, d, dtype=torch.float64, device="cuda")
+    lse = torch.full((b, hq, sq), -math.inf, dtype=torch.float64, device="cuda")
+    for i in range(b):
+        for h in range(hq):
+            kh, vh = k[i, :, h // group].double(), v[i, :, h // group].double()
+            for s0 in range(0, sq, chunk):
+                s1 = min(s0 + chunk, sq)
+                n, hidden = _visible(case, s0, s1, q_off, sk)
+                if n == 0:
+                    continue
+                s = (q[i, s0:s1, h].double() @ kh[:n].T).mul_(SCALE)
+                if hidden is not None:
+                    s.masked_fill_(hidden, -math.inf)
+                part = torch.logsumexp(s, dim=1)
+                lse[i, h, s0:s1] = part
+                p = s.sub_(part[:, None]).exp_().nan_to_num_(0.0)
+                o[i, s0:s1, h] = p @ vh[:n]
+    return o, lse
+
+
+def _exact_backward(case, dout, q, k, v, o, lse, q_off, chunk=2048):
+    """dq, dk, dv and rowsum(dout * o) [B,H,S] in fp64, given the forward's o and lse."""
+    b, sq, hq, d = q.shape
+    sk, group = k.shape[1], hq // k.shape[2]
+    dq = torch.zeros(b, sq, hq, d, dtype=torch.float64, device="cuda")
+    dk = torch.zeros(b, sk, hq // group, d, dtype=torch.float64, device="cuda")
+    dv = torch.zeros_like(dk)
+    delta = (dout.double() * o.double()).sum(-1).transpose(1, 2).contiguous()
+    for i in range(b):
+        for h in range(hq):
+            kh, vh = k[i, :, h // group].double(), v[i, :, h // group].double()
+            for s0 in range(0, sq, chunk):
+                s1 = min(s0 + chunk, sq)
+                n, hidden = _visible(case, s0, s1, q_off, sk)
+                if n == 0:
+                    continue
+                qh, gh = q[i, s0:s1, h].double(), dout[i, s0:s1, h].double()
+                p = (qh @ kh[:n].T).mul_(SCALE).sub_(lse[i, h, s0:s1, None].double()).exp_()
+                if hidden is not None:
+                    p.masked_fill_(hidden, 0.0)
+                dv[i, :n, h // group] += p.T @ gh
+                ds = (gh @ vh[:n].T).sub_(delta[i, h, s0:s1, None]).mul_(p).mul_(SCALE)
+                dq[i, s0:s1, h] = ds @ kh[:n]
+                dk[i, :n, h // group] += ds.T @ qh
+    return dq, torch.stack((dk, dv)), delta
+
+
+def exact(case, seed):
+    """What run() returns, by plain attention in fp64 on the same inputs; None where that would take too long."""
+    if work(case)["flops"] > 4.0e13:
+        return None
+    s, kind = prepare(case, seed), case["kind"]
+    if kind in ("forward", "train"):
+        o, lse = _exact_forward(case, s["q"], s["kv"][0], s["kv"][1], 0)
+        if kind == "forward":
+            return o, lse
+        dq, dkv, _ = _exact_backward(case, s["dout"], s["q"], s["kv"][0], s["kv"][1], o, lse, 0)
+        return o, lse, dq, dkv
+    if kind in ("segments", "steps"):
+        # the shards in sequence order: the result does not depend on the order of arrival
+        kv = torch.cat(s["kv"], dim=2)
+        o, lse = _exact_forward(case, s["q"], kv[0], kv[1], s["rank"] * s["shard"])
+        return (o, lse.transpose(1, 2).unsqueeze(-1)) if kind == "steps" else (o, lse)
+    q_off = case["sk"] - case["sq"]
+    if kind == "block":
+        return _exact_forward(case, s["q"], s["k"], s["v"], q_off)
+    return _exact_backward(case, s["dout"], s["q"], s["k"], s["v"], s["o"], s["lse"], q_off)
+
+
 def _pairs(sq, sk, q_off, causal):
     """Visible (query, key) pairs of one head; key j is visible to query i iff j <= q_off + i."""
     if not causal:
