@@ -79,6 +79,14 @@ typedef struct mb_attn_fwd_args {
  * A row that sees no key gets o = 0 and lse = -inf. */
 MB_API int mb_attn_fwd(const mb_attn_fwd_args* args, void* cuda_stream);
 
+/* mb_attn_fwd with scratch.  Shapes whose query tiles leave SMs idle (few rows against many keys, or a partly
+ * filled last wave) are then split over their keys: the shares' rows, maxima and sums go through the
+ * workspace in fp32 and a second kernel merges them.  mb_attn_fwd_workspace returns the bytes that the call
+ * can use on the current device (0: none).  The workspace (16-byte aligned, contents arbitrary) belongs to
+ * the call until its work on the stream is done; a smaller one, or NULL, runs the call unsplit. */
+MB_API int64_t mb_attn_fwd_workspace(const mb_attn_fwd_args* args);
+MB_API int mb_attn_fwd_ws(const mb_attn_fwd_args* args, void* workspace, uint64_t workspace_bytes, void* cuda_stream);
+
 /* One query shard of a multi-shard forward launch, with where its results go. */
 typedef struct mb_fwd_job {
   const void* q; /* [batch, sq, hq, head_dim] */

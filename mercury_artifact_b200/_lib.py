@@ -297,9 +297,14 @@ class MercuryB200Error(RuntimeError):
     pass
 
 
+# entry points that return something other than an MB_* code
+_RESTYPES = {"mb_attn_fwd_workspace": C.c_int64}
+
 _SIGNATURES = {
     "mb_version": [],
     "mb_attn_fwd": [C.POINTER(AttnFwdArgs), C.c_void_p],
+    "mb_attn_fwd_workspace": [C.POINTER(AttnFwdArgs)],
+    "mb_attn_fwd_ws": [C.POINTER(AttnFwdArgs), C.c_void_p, C.c_uint64, C.c_void_p],
     "mb_attn_fwd_multi": [C.POINTER(AttnFwdMultiArgs), C.c_void_p],
     "mb_attn_bwd_preprocess": [C.POINTER(BwdPreprocessArgs), C.c_void_p],
     "mb_attn_bwd": [C.POINTER(AttnBwdArgs), C.c_void_p],
@@ -334,7 +339,7 @@ def _bind(path: Path) -> C.CDLL:
     try:
         for name, argtypes in _SIGNATURES.items():
             fn = getattr(handle, name)  # AttributeError: the shared object predates this binding
-            fn.restype = C.c_int
+            fn.restype = _RESTYPES.get(name, C.c_int)
             fn.argtypes = argtypes
     except AttributeError:
         import _ctypes

@@ -104,7 +104,12 @@ def attn_fwd_segments(
         seg.ready_value = int(flag_value)
     args.hkv = hkv if hkv is not None else hq
     with torch.cuda.device(q.device):
-        _lib.check(_lib.lib.mb_attn_fwd(C.byref(args), C.c_void_p(_stream_ptr())), "mb_attn_fwd")
+        # scratch of a launch that splits items over their keys (results in another GPU's memory are written by
+        # the attention kernel itself); freed in stream order by the caching allocator
+        need = 0 if raw else _lib.lib.mb_attn_fwd_workspace(C.byref(args))
+        ws = torch.empty(need, dtype=torch.uint8, device=q.device) if need > 0 else None
+        _lib.check(_lib.lib.mb_attn_fwd_ws(C.byref(args), ws.data_ptr() if need > 0 else None, need,
+                                           C.c_void_p(_stream_ptr())), "mb_attn_fwd_ws")
     return (None, None) if raw else (out, lse)
 
 

@@ -51,15 +51,26 @@ __device__ __forceinline__ int seg_tiles(const FwdSmem* ctl, int s) {
 }
 __device__ __forceinline__ TileIter iter_first(const FwdSmem* ctl, int nseg) {
   TileIter it{0, 0};
-  while (it.s < nseg && seg_tiles(ctl, it.s) == 0) ++it.s;
+  while (it.s < nseg && seg_tiles(ctl, it.s) <= ctl->t_lo[it.s]) ++it.s;
+  if (it.s < nseg) it.jt = ctl->t_lo[it.s];
   return it;
 }
 __device__ __forceinline__ void iter_next(const FwdSmem* ctl, int nseg, TileIter& it) {
   if (++it.jt >= seg_tiles(ctl, it.s)) {
-    it.jt = 0;
     ++it.s;
-    while (it.s < nseg && seg_tiles(ctl, it.s) == 0) ++it.s;
+    while (it.s < nseg && seg_tiles(ctl, it.s) <= ctl->t_lo[it.s]) ++it.s;
+    it.jt = it.s < nseg ? ctl->t_lo[it.s] : 0;
   }
+}
+
+// Query tile pair, head and batch entry of a job's work item: batch entry by batch entry and head by head,
+// heavier (later) query rows first when causal.
+struct ItemCoords {
+  int pair, h, b;
+};
+__device__ __forceinline__ ItemCoords item_coords(int item, int n_pairs, int Hq, int causal) {
+  const int pidx = item % n_pairs, bh = item / n_pairs;
+  return ItemCoords{causal ? n_pairs - 1 - pidx : pidx, bh % Hq, bh / Hq};
 }
 
 // Register budgets.  setmaxnreg can only redistribute the registers the CTA was launched with
@@ -95,12 +106,18 @@ attn_fwd_kernel(const __grid_constant__ FwdMaps maps, const __grid_constant__ Fw
     ctl->job = a.job[jid];
     // CTAs are dispatched in grid order: job by job, inside a job batch entry by batch entry and head by
     // head (the CTAs running at one time share a few heads' K/V through L2), heavier query rows first.
-    const int local = (int)blockIdx.x - a.job[jid].x_begin;
-    const int np = a.job[jid].n_pairs;
-    const int pidx = local % np;
-    ctl->pair = a.causal ? (np - 1 - pidx) : pidx;
-    ctl->h = (local / np) % a.Hq;
-    ctl->b = (local / np) / a.Hq;
+    int local = (int)blockIdx.x - a.job[jid].x_begin;
+    ctl->slot = -1;
+    ctl->part = 0;
+    if (local >= a.split_begin) {
+      ctl->slot = local - a.split_begin;
+      ctl->part = ctl->slot % a.nsplit;
+      local = a.split_begin + ctl->slot / a.nsplit;
+    }
+    const ItemCoords it = item_coords(local, a.job[jid].n_pairs, a.Hq, a.causal);
+    ctl->pair = it.pair;
+    ctl->h = it.h;
+    ctl->b = it.b;
   }
   __syncthreads();
   const FwdJob& J = ctl->job;
@@ -126,13 +143,37 @@ attn_fwd_kernel(const __grid_constant__ FwdMaps maps, const __grid_constant__ Fw
     fence_barrier_init();
     fence_proxy_async_smem();
   }
-  // K/V tiles of each segment that each of the two query tiles takes part in: one thread per entry
+  // K/V tiles of each segment that each of the two query tiles takes part in: one lane per segment
   // (computed by one thread this was ~4 000 cycles of a CTA's prologue at 32 segments)
-  if (tid < 2 * MB_MAX_SEGMENTS) {
-    const int i = tid / MB_MAX_SEGMENTS, s = tid % MB_MAX_SEGMENTS;
-    ctl->n_tiles[i][s] = (s < a.nseg && ((J.seg_mask >> s) & 1u))
-                             ? visible_tiles(q0 + i * kBM, J.Sq, J.q_off, a.causal, a.seg_sk[s], a.seg_koff[s])
-                             : 0;
+  static_assert(MB_MAX_SEGMENTS == 32, "one lane of warp 0 per segment");
+  if (warp == 0) {
+    int n[2] = {0, 0};
+    if (lane < a.nseg && ((J.seg_mask >> lane) & 1u)) {
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+        n[i] = visible_tiles(q0 + i * kBM, J.Sq, J.q_off, a.causal, a.seg_sk[lane], a.seg_koff[lane]);
+    }
+    int lo = 0;
+    if (ctl->slot >= 0) {
+      // This CTA's share of the item's walk over all its K/V tiles: an equal part, cut at whole tiles.
+      const int mine = max(n[0], n[1]);
+      int incl = mine;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const int up = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= d) incl += up;
+      }
+      const long long all = __shfl_sync(0xffffffffu, incl, 31);
+      const int before = incl - mine;
+      const int first = (int)(all * ctl->part / a.nsplit), last = (int)(all * (ctl->part + 1) / a.nsplit);
+      lo = min(max(first - before, 0), mine);
+      const int hi = min(max(last - before, 0), mine);
+      n[0] = min(n[0], hi);
+      n[1] = min(n[1], hi);
+    }
+    ctl->t_lo[lane] = lo;
+    ctl->n_tiles[0][lane] = n[0];
+    ctl->n_tiles[1][lane] = n[1];
   }
   if (warp == 8) {
     tmem_alloc(&ctl->tmem_base, 512);
@@ -145,7 +186,7 @@ attn_fwd_kernel(const __grid_constant__ FwdMaps maps, const __grid_constant__ Fw
   const uint32_t tmem = ctl->tmem_base;  // columns: S [0,128) P0 [128,192) P1 [192,256) O0 [256,384) O1 [384,512)
 
   bool any_work = false;
-  for (int s = 0; s < a.nseg; ++s) any_work |= (ctl->n_tiles[0][s] | ctl->n_tiles[1][s]) != 0;
+  for (int s = 0; s < a.nseg; ++s) any_work |= seg_tiles(ctl, s) > ctl->t_lo[s];
 
   // Registers move from the auxiliary warpgroup (warps 8-11) to the two softmax
   // warpgroups; each role changes its own budget as the first thing it does.
@@ -178,7 +219,7 @@ attn_fwd_kernel(const __grid_constant__ FwdMaps maps, const __grid_constant__ Fw
       const int b_ = ctl->b, hkv = ctl->h / a.group;
       // One K or V tile into the next stage of the ring.
       auto load_tile = [&](int which, const TileIter& it) {
-        if (which == 0 && it.jt == 0 && a.seg_flag[it.s] != nullptr) {
+        if (which == 0 && it.jt == ctl->t_lo[it.s] && a.seg_flag[it.s] != nullptr) {
           // The shard is being staged by another stream: wait (bounded) for its arrival flag,
           // then order the TMA reads (async proxy) after the flag read.
           ok = flag_wait_ge(a.seg_flag[it.s], a.seg_flag_value[it.s], abort_word, MB_ERR_TIMEOUT_SEGMENT,
@@ -232,7 +273,7 @@ attn_fwd_kernel(const __grid_constant__ FwdMaps maps, const __grid_constant__ Fw
     if (any_work) {  // whole warp, converged
       constexpr uint32_t kStageUnits = kTileBytes / 16;
       int total = 0;  // K/V tiles this CTA walks through
-      for (int s = 0; s < a.nseg; ++s) total += seg_tiles(ctl, s);
+      for (int s = 0; s < a.nseg; ++s) total += max(seg_tiles(ctl, s) - ctl->t_lo[s], 0);
       bool ok = true;
       if (warp == 8) {
         constexpr uint32_t idesc_qk = umma_idesc_bf16(kBM, kBN, false, false);
@@ -244,7 +285,7 @@ attn_fwd_kernel(const __grid_constant__ FwdMaps maps, const __grid_constant__ Fw
         for (int s = 0; s < a.nseg && ok; ++s) {
           const int n0 = ctl->n_tiles[0][s], n1 = ctl->n_tiles[1][s];
           const int nmax = max(n0, n1);
-          for (int jt = 0; jt < nmax && ok; ++jt, ++g) {
+          for (int jt = ctl->t_lo[s]; jt < nmax && ok; ++jt, ++g) {
             const int pos = g == 0 ? 0 : 2 * g - 1;
             const int stage = pos % kFwdStages;
             ok = mbar_wait_warp(&ctl->kv_full[stage], (pos / kFwdStages) & 1, abort_word, MB_ERR_TIMEOUT_KV_FULL, a.wait_cycles);
@@ -275,7 +316,7 @@ attn_fwd_kernel(const __grid_constant__ FwdMaps maps, const __grid_constant__ Fw
         for (int s = 0; s < a.nseg && ok; ++s) {
           const int n0 = ctl->n_tiles[0][s], n1 = ctl->n_tiles[1][s];
           const int nmax = max(n0, n1);
-          for (int jt = 0; jt < nmax && ok; ++jt, ++g) {
+          for (int jt = ctl->t_lo[s]; jt < nmax && ok; ++jt, ++g) {
             const int pos = g == total - 1 ? 2 * total - 1 : 2 * g + 2;
             const int stage = pos % kFwdStages;
             ok = mbar_wait_warp(&ctl->kv_full[stage], (pos / kFwdStages) & 1, abort_word, MB_ERR_TIMEOUT_KV_FULL, a.wait_cycles);
@@ -372,7 +413,7 @@ attn_fwd_kernel(const __grid_constant__ FwdMaps maps, const __grid_constant__ Fw
       const int nt = ctl->n_tiles[i][s];
       const int sk = a.seg_sk[s];
       const int koff = a.seg_koff[s];
-      for (int jt = 0; jt < nt; ++jt) {
+      for (int jt = ctl->t_lo[s]; jt < nt; ++jt) {
         ok = mbar_wait_warp(&ctl->s_full[i], cnt & 1, abort_word, MB_ERR_TIMEOUT_S, a.wait_cycles);
         if (!ok) break;
         tc_fence_after();
@@ -491,7 +532,25 @@ attn_fwd_kernel(const __grid_constant__ FwdMaps maps, const __grid_constant__ Fw
       if (ok) {
         const bool store = qrow < J.Sq;
         if (have_acc) tc_fence_after();
-        if (J.st_out) {
+        if (ctl->slot >= 0) {
+          // a share of the item: rows as they are, column group by column group (contiguous over a warp)
+          const int r = i * kBM + row;
+          if (cnt > 0) {
+            float4* dst = a.part_o + (long long)ctl->slot * (32 * 2 * kBM) + r;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              uint32_t orow[32];
+              tmem_ld32(tOi + c * 32, orow);
+              tmem_wait_ld();
+#pragma unroll
+              for (int v = 0; v < 8; ++v)
+                dst[(c * 8 + v) * (2 * kBM)] =
+                    make_float4(__uint_as_float(orow[v * 4 + 0]), __uint_as_float(orow[v * 4 + 1]),
+                                __uint_as_float(orow[v * 4 + 2]), __uint_as_float(orow[v * 4 + 3]));
+            }
+          }
+          a.part_ml[ctl->slot * (2 * kBM) + r] = make_float2(m_ref, l);
+        } else if (J.st_out) {
           float4* dst = reinterpret_cast<float4*>(J.st_o + st_row * kD);
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
@@ -581,8 +640,172 @@ attn_fwd_kernel(const __grid_constant__ FwdMaps maps, const __grid_constant__ Fw
 }
 
 // ---------------------------------------------------------------------------
+// split items: the shares of an item become its result
+// ---------------------------------------------------------------------------
+struct FwdMergeArgs {
+  const float4* part_o;  // [slot][32 column groups][256 rows]
+  const float2* part_ml;
+  __nv_bfloat16* o;
+  long long o_sb, o_ss, o_sh;
+  float* lse;
+  long long lse_sb, lse_sh;
+  int Sq, Hq, n_pairs, causal, first_item, nsplit;
+  float scale, scale_log2;
+};
+
+// o = sum_p w_p O_p / sum_p w_p l_p with w_p = exp(scale * (m_p - max m)), in fp32.  A warp handles 32 rows and
+// 16 of the 128 columns, so every load of a share is 512 contiguous bytes; a thread's 16 bf16 results are one
+// 32-byte sector.  Latency-bound: the shares are in L2, and a launch has at most a few blocks per SM.
+__global__ void __launch_bounds__(256) fwd_split_merge_kernel(const FwdMergeArgs a) {
+  constexpr int kRows = 2 * kBM;
+  const int lane = threadIdx.x & 31, group = threadIdx.x >> 5;  // column group: 16 columns
+  const int item = blockIdx.x;
+  const int r = blockIdx.y * 32 + lane;
+  const ItemCoords it = item_coords(a.first_item + item, a.n_pairs, a.Hq, a.causal);
+  const int qrow = it.pair * kRows + r;
+  if (qrow >= a.Sq) return;
+  const long long slot0 = (long long)item * a.nsplit;
+  const float2* ml = a.part_ml + slot0 * kRows + r;
+  float m = -INFINITY;
+#pragma unroll 4
+  for (int p = 0; p < a.nsplit; ++p) m = fmaxf(m, ml[p * kRows].x);
+  float l = 0.f;
+  float acc[16];
+#pragma unroll
+  for (int e = 0; e < 16; ++e) acc[e] = 0.f;
+  const float4* src = a.part_o + (slot0 * 32 + group * 4) * kRows + r;
+#pragma unroll 4
+  for (int p = 0; p < a.nsplit; ++p) {
+    const float2 s = ml[p * kRows];
+    const bool has = !(s.y == 0.f);  // a share without visible keys has stored no rows
+    float4 x[4];
+#pragma unroll
+    for (int v = 0; v < 4; ++v)
+      x[v] = has ? src[((long long)p * 32 + v) * kRows] : make_float4(0.f, 0.f, 0.f, 0.f);
+    const float w = has ? fast_exp2((s.x - m) * a.scale_log2) : 0.f;
+    l = fmaf(w, s.y, l);
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      acc[v * 4 + 0] = fmaf(w, x[v].x, acc[v * 4 + 0]);
+      acc[v * 4 + 1] = fmaf(w, x[v].y, acc[v * 4 + 1]);
+      acc[v * 4 + 2] = fmaf(w, x[v].z, acc[v * 4 + 2]);
+      acc[v * 4 + 3] = fmaf(w, x[v].w, acc[v * 4 + 3]);
+    }
+  }
+  const float inv = l > 0.f ? 1.f / l : 0.f;
+  uint4* dst = reinterpret_cast<uint4*>(a.o + it.b * a.o_sb + qrow * a.o_ss + it.h * a.o_sh + group * 16);
+#pragma unroll
+  for (int v = 0; v < 2; ++v) {
+    uint4 w;
+    w.x = pack_bf16x2(acc[v * 8 + 0] * inv, acc[v * 8 + 1] * inv);
+    w.y = pack_bf16x2(acc[v * 8 + 2] * inv, acc[v * 8 + 3] * inv);
+    w.z = pack_bf16x2(acc[v * 8 + 4] * inv, acc[v * 8 + 5] * inv);
+    w.w = pack_bf16x2(acc[v * 8 + 6] * inv, acc[v * 8 + 7] * inv);
+    dst[v] = w;
+  }
+  if (group == 0) a.lse[it.b * a.lse_sb + it.h * a.lse_sh + qrow] = l > 0.f ? m * a.scale + __logf(l) : -INFINITY;
+}
+
+// ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
+// How a single-job launch is cut: items before split_begin run whole, the others as nsplit shares each.
+struct FwdSplit {
+  int split_begin, nsplit, slots;
+};
+constexpr size_t kSlotBytes = 2 * kBM * (kD * sizeof(float) + sizeof(float2));
+
+static int sm_count() {
+  static int count[64] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  if (count[dev] == 0) {
+    int n = 0;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
+    count[dev] = n;
+  }
+  return count[dev];
+}
+
+// Without a split a launch of few items runs on as many SMs as it has items, and a last wave of few items leaves the
+// others idle.  Measured (B200): 100 queries against 16 384 keys, 32 heads over 8 K/V heads, 164 us whole, 55 us in
+// 4 shares; 4 096 queries against 32 768 keys, 32 heads (3.46 waves), 1.89 ms whole, 1.76 ms with the last
+// 68 items in 2 shares.  The price of a split is one CTA start per share and one launch that merges.
+static FwdSplit plan_split(const mb_attn_fwd_args* x) {
+  const FwdSplit whole{INT_MAX, 1, 0};
+  if (x->sq <= 0 || x->softmax_scale <= 0.f) return whole;
+  const int sms = sm_count();
+  const int np = (x->sq + 2 * kBM - 1) / (2 * kBM), heads = x->hq;
+  const long long items = (long long)np * heads * x->batch;
+  if (sms <= 0 || items > INT_MAX) return whole;
+  // A launch over several shards is cut in its last wave only: smaller ones add up in the order of the chained
+  // jobs of mb_attn_fwd_multi, whose results they equal bit for bit.
+  if (x->nseg > 1 && (x->causal || items < sms)) return whole;
+  for (int s = 0; s < x->nseg; ++s)
+    if (x->seg[s].ready_flag != nullptr) return whole;
+  // K/V tiles of the longest item, of the shortest one and of all items of a head
+  long long t_max = 0, t_min = 0, t_sum = 0;
+  for (int s = 0; s < x->nseg; ++s) t_max += (max(x->seg[s].sk, 0) + kBN - 1) / kBN;
+  if (x->causal) {
+    if (items > 4ll * sms) return whole;
+    t_min = t_max;
+    t_max = 0;
+    for (int p = 0; p < np; ++p) {
+      long long t = 0;
+      const long long last = (long long)x->q_off + min((p + 1) * 2 * kBM - 1, x->sq - 1);
+      for (int s = 0; s < x->nseg; ++s) {
+        const long long vis = min((long long)x->seg[s].sk, last - x->seg[s].k_off + 1);
+        if (vis > 0) t += (vis + kBN - 1) / kBN;
+      }
+      t_max = max(t_max, t);
+      t_min = min(t_min, t);
+      t_sum += t;
+    }
+  }
+  // Costs in steps of one K/V tile against both query tiles (about 1.6 us): starting and ending a CTA, and
+  // the extra launch that merges the shares.
+  constexpr double kCta = 2.0, kMerge = 3.0;
+  constexpr int kMaxSplit = 32;
+  const long long slot_cap = 3ll * sms;
+  FwdSplit best = whole;
+  if (x->causal) {
+    // Items of unequal length, longest first: one after the other on every SM until the shortest ones fill up
+    // the end, unless there are fewer items than SMs.
+    const double total = (double)t_sum * heads * x->batch;
+    auto cost = [&](int ns) {
+      const double longest = (double)((t_max + ns - 1) / ns) + kCta;
+      if (items * ns <= sms) return longest;
+      return max(longest, (total + items * ns * kCta) / sms + (double)t_min / ns + kCta);
+    };
+    double t_best = cost(1);
+    for (int ns = 2; ns <= kMaxSplit && ns <= t_max && items * ns <= slot_cap; ++ns) {
+      const double t = cost(ns) + kMerge;
+      if (t < t_best) {
+        t_best = t;
+        best = FwdSplit{0, ns, (int)(items * ns)};
+      }
+    }
+  } else {
+    // Equal items: whole waves run as they are, the items of the last, partly filled one are split.
+    const int rest = (int)(items % sms);
+    double t_best = t_max + kCta;
+    for (int ns = 2; rest > 0 && ns <= kMaxSplit && ns <= t_max && (long long)rest * ns <= slot_cap; ++ns) {
+      const int waves = (rest * ns + sms - 1) / sms;
+      const double t = waves * ((double)((t_max + ns - 1) / ns) + kCta) + kMerge;
+      if (t < t_best) {
+        t_best = t;
+        best = FwdSplit{(int)(items - rest), ns, rest * ns};
+      }
+    }
+  }
+  return best;
+}
+
+long long attn_fwd_workspace(const mb_attn_fwd_args* x) {
+  if (x == nullptr || x->nseg < 0 || x->nseg > MB_MAX_SEGMENTS || x->hq <= 0 || x->batch <= 0) return 0;
+  return plan_split(x).slots * (long long)kSlotBytes;
+}
+
 static int make_tile_map(CUtensorMap* map, const void* ptr, int D, int H, int S, int B, long long sb, long long ss,
                          long long sh) {
   cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)H, (cuuint64_t)S, (cuuint64_t)B};
@@ -600,7 +823,7 @@ void set_peer_wait_ms(unsigned ms) { g_peer_wait_ms = ms == 0 ? 1 : ms; }
 // 2e6 cycles per millisecond is at least the requested time.
 long long peer_wait_cycles() { return g_peer_wait_ms * 2000000LL; }
 
-int launch_attn_fwd_multi(const mb_attn_fwd_multi_args* x, cudaStream_t stream) {
+static int launch_fwd(const mb_attn_fwd_multi_args* x, const FwdSplit& split, void* ws, cudaStream_t stream) {
   if (x == nullptr) return MB_E_INVALID;
   if (x->head_dim != kD) return MB_E_UNSUPPORTED;
   if (x->batch <= 0 || x->hq <= 0 || x->hkv <= 0 || x->hq % x->hkv != 0) return MB_E_INVALID;
@@ -722,13 +945,39 @@ int launch_attn_fwd_multi(const mb_attn_fwd_multi_args* x, cudaStream_t stream) 
   a.status = x->status ? x->status : default_status_word();
   if (a.status == nullptr) return MB_E_CUDA;
 
+  a.split_begin = split.split_begin;
+  a.nsplit = split.nsplit;
+  if (split.slots > 0) {
+    a.part_o = static_cast<float4*>(ws);
+    a.part_ml = reinterpret_cast<float2*>(a.part_o + (size_t)split.slots * (2 * kBM * kD / 4));
+    x_total = split.split_begin + split.slots;
+  }
   dim3 grid(x_total, 1, 1);
   attn_fwd_kernel<<<grid, kFwdThreads, kFwdSmemBytes, stream>>>(maps, a);
-  return cuda_ok(cudaGetLastError(), "launch attn_fwd_kernel") ? MB_SUCCESS : MB_E_CUDA;
+  if (!cuda_ok(cudaGetLastError(), "launch attn_fwd_kernel")) return MB_E_CUDA;
+  if (split.slots > 0) {
+    const FwdJob& J = a.job[0];
+    FwdMergeArgs m;
+    m.part_o = a.part_o; m.part_ml = a.part_ml;
+    m.o = J.o; m.o_sb = J.o_sb; m.o_ss = J.o_ss; m.o_sh = J.o_sh;
+    m.lse = J.lse; m.lse_sb = J.lse_sb; m.lse_sh = J.lse_sh;
+    m.Sq = J.Sq; m.Hq = a.Hq; m.n_pairs = J.n_pairs; m.causal = a.causal;
+    m.first_item = split.split_begin; m.nsplit = split.nsplit;
+    m.scale = a.scale; m.scale_log2 = a.scale_log2;
+    const int rows = min(2 * kBM, J.Sq);  // a job shorter than one item has no rows past Sq
+    fwd_split_merge_kernel<<<dim3(split.slots / split.nsplit, (rows + 31) / 32), 256, 0, stream>>>(m);
+    if (!cuda_ok(cudaGetLastError(), "launch fwd_split_merge_kernel")) return MB_E_CUDA;
+  }
+  return MB_SUCCESS;
 }
 
-// One query shard: the single-job form of the launch above.
-int launch_attn_fwd(const mb_attn_fwd_args* x, cudaStream_t stream) {
+int launch_attn_fwd_multi(const mb_attn_fwd_multi_args* x, cudaStream_t stream) {
+  return launch_fwd(x, FwdSplit{INT_MAX, 1, 0}, nullptr, stream);
+}
+
+// One query shard: the single-job form of the launch above.  With a workspace of attn_fwd_workspace(x) bytes the
+// launch may split items over their keys; with less (or none) it runs them whole.
+int launch_attn_fwd(const mb_attn_fwd_args* x, void* ws, unsigned long long ws_bytes, cudaStream_t stream) {
   if (x == nullptr) return MB_E_INVALID;
   if (x->nseg < 0 || x->nseg > MB_MAX_SEGMENTS) return MB_E_INVALID;
   if (x->sq < 0) return MB_E_INVALID;
@@ -749,7 +998,13 @@ int launch_attn_fwd(const mb_attn_fwd_args* x, cudaStream_t stream) {
   j.sq = x->sq; j.q_off = x->q_off;
   for (int s = 0; s < x->nseg; ++s) m.seg[s] = x->seg[s];
   m.status = x->status;
-  return launch_attn_fwd_multi(&m, stream);
+  FwdSplit split{INT_MAX, 1, 0};
+  if (ws != nullptr && x->batch > 0 && x->hq > 0) {
+    split = plan_split(x);
+    if (split.slots * (unsigned long long)kSlotBytes > ws_bytes || (reinterpret_cast<uintptr_t>(ws) & 15u))
+      split = FwdSplit{INT_MAX, 1, 0};
+  }
+  return launch_fwd(&m, split, ws, stream);
 }
 
 }  // namespace mb

@@ -67,6 +67,13 @@ struct FwdArgs {
   long long peer_wait_cycles;  // budget of a wait for data another GPU delivers
   long long wait_cycles;       // budget of a wait inside the CTA (plus the above when the launch has flags)
   int* status;
+  // Work items whose keys are split over several CTAs (single-job launches without flags): the first
+  // `split_begin` CTAs take one item each, the others `nsplit` CTAs per item.  Split CTA c leaves its
+  // unnormalised rows in slot c - split_begin of `part_o` ([slot][32 column groups][256 rows] of float4, so
+  // that the stores of a warp are contiguous) and their (maximum, sum) pairs in `part_ml` ([slot][256]).
+  int split_begin, nsplit;
+  float4* part_o;
+  float2* part_ml;
 };
 
 struct FwdSmem {
@@ -82,7 +89,11 @@ struct FwdSmem {
   int abort_word;
   int jid;
   int pair, h, b;  // this CTA's query tile pair, head and batch entry
-  int n_tiles[2][MB_MAX_SEGMENTS];  // K/V tiles of each segment that query tile i takes part in
+  int part;        // which share of a split item this CTA has
+  int slot;        // where a split item's CTA leaves its state (-1: the CTA has the item to itself)
+  // K/V tiles of each segment that query tile i takes part in: t_lo <= tile < n_tiles (this CTA's share)
+  int n_tiles[2][MB_MAX_SEGMENTS];
+  int t_lo[MB_MAX_SEGMENTS];
   FwdJob job;                       // this CTA's job (a copy: read with fixed offsets, no registers held)
 };
 

@@ -61,7 +61,13 @@ int mb_last_cuda_error(char* buf, int32_t len) {
 }
 
 int mb_attn_fwd(const mb_attn_fwd_args* args, void* cuda_stream) {
-  return mb::launch_attn_fwd(args, static_cast<cudaStream_t>(cuda_stream));
+  return mb::launch_attn_fwd(args, nullptr, 0, static_cast<cudaStream_t>(cuda_stream));
+}
+
+int64_t mb_attn_fwd_workspace(const mb_attn_fwd_args* args) { return mb::attn_fwd_workspace(args); }
+
+int mb_attn_fwd_ws(const mb_attn_fwd_args* args, void* workspace, uint64_t workspace_bytes, void* cuda_stream) {
+  return mb::launch_attn_fwd(args, workspace, workspace_bytes, static_cast<cudaStream_t>(cuda_stream));
 }
 
 int mb_attn_fwd_multi(const mb_attn_fwd_multi_args* args, void* cuda_stream) {

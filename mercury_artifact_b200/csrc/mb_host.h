@@ -19,7 +19,8 @@ bool cuda_ok(cudaError_t e, const char* what);
 // Device address of the library's status word on the current device (nullptr on failure).
 int* default_status_word();
 
-int launch_attn_fwd(const mb_attn_fwd_args* args, cudaStream_t stream);
+int launch_attn_fwd(const mb_attn_fwd_args* args, void* ws, unsigned long long ws_bytes, cudaStream_t stream);
+long long attn_fwd_workspace(const mb_attn_fwd_args* args);
 int launch_attn_fwd_multi(const mb_attn_fwd_multi_args* args, cudaStream_t stream);
 
 // Budget of in-kernel waits for data that other GPUs deliver (mb_set_peer_wait_ms), in SM cycles.

@@ -378,3 +378,57 @@ def test_eight_chains_of_one_launch_like_one_rank_of_eight(causal):
         ro, rl = mb.attn_fwd_segments(q[:, j * L:(j + 1) * L], segs, scale, causal=causal, q_off=j * L)
         assert torch.equal(o[:, j * L:(j + 1) * L], ro), j
         assert torch.equal(lse[:, :, j * L:(j + 1) * L], rl), j
+
+
+SPLIT_CASES = [
+    # B, Sq, Sk, Hq, Hkv, causal, q_off, K/V shards, does the launch split items over their keys
+    (1, 1, 3001, 8, 2, False, 0, 1, True),        # one query, four heads to a tile
+    (1, 100, 4096, 8, 2, True, 3996, 1, True),    # shares of a causal item; heads packed
+    (2, 77, 2500, 16, 4, True, 2423, 1, True),    # ragged everywhere
+    (1, 300, 2049, 4, 4, False, 0, 1, True),      # more queries than one item, last key tile of one key
+    (1, 700, 1600, 8, 8, True, 0, 1, True),       # early rows: shares without a visible key
+    (1, 1300, 900, 2, 2, True, -300, 1, True),    # rows without any visible key in every share
+    (1, 33, 1500, 6, 2, False, 0, 1, True),       # a group that does not divide a tile: heads apart
+    (1, 65, 300, 128, 1, True, 235, 1, False),    # the largest group that fits a tile; too few keys to split
+    (3, 6390, 1400, 2, 2, False, 0, 1, True),     # 150 items: the last two split, the first 148 whole
+    (3, 6390, 1400, 2, 2, False, 0, 3, True),     # the same over three shards
+    (2, 300, 1400, 4, 2, True, 1100, 3, False),   # several shards, less than a wave: whole
+]
+
+
+@pytest.mark.parametrize("B,Sq,Sk,Hq,Hkv,causal,q_off,shards,splits", SPLIT_CASES)
+def test_items_split_over_their_keys_match_oracle(B, Sq, Sk, Hq, Hkv, causal, q_off, shards, splits, monkeypatch):
+    """Launches that share a work item between CTAs (and merge the shares), and tiles that hold the rows of all
+    heads of a group.  The shares are merged in fp32, so the tolerance is the one of the unsplit kernel."""
+    import mercury_artifact_b200 as mb
+    from mercury_artifact_b200 import _lib
+    from oracle import block
+
+    q, k, v, _ = seeded_qkv(11, B, max(Sq, Sk), Hq, Hkv, 128)
+    q, k, v = q[:, :Sq], k[:, :Sk], v[:, :Sk]
+    scale = 128 ** -0.5
+    need = []
+    real_lib = _lib.lib
+
+    class Lib:
+        def __getattr__(self, name):
+            return getattr(real_lib, name)
+
+        def mb_attn_fwd_workspace(self, args):
+            need.append(real_lib.mb_attn_fwd_workspace(args))
+            return need[-1]
+
+    monkeypatch.setattr(_lib, "lib", Lib())
+    qd, kd, vd = q.cuda(), k.cuda(), v.cuda()
+    cut = [Sk * i // shards for i in range(shards + 1)]
+    segs = [(kd[:, a:b], vd[:, a:b], a) for a, b in zip(cut[:-1], cut[1:])]
+    o, lse = mb.attn_fwd_segments(qd, segs, scale, causal=causal, q_off=q_off)
+    monkeypatch.undo()
+    _status_ok()
+    assert (need[0] > 0) == splits
+    rows = slice(0, Sq) if Sq < 5000 else slice(Sq - 700, Sq)   # the long case: rows of whole and of split items
+    ro, rl = block.block_attn_fwd(q[:, rows], k, v, scale, causal=causal, q_off=q_off)
+    _check(o[:, rows], lse[:, :, rows], ro, rl)
+    if Sq >= 5000:
+        ro, rl = block.block_attn_fwd(q[:, :300], k, v, scale)
+        _check(o[:, :300], lse[:, :, :300], ro, rl)
