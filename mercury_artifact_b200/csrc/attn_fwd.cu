@@ -63,13 +63,16 @@ __device__ __forceinline__ void iter_next(const FwdSmem* ctl, int nseg, TileIter
   }
 }
 
-// Query tile pair, head and batch entry of a job's work item: batch entry by batch entry and head by head,
-// heavier (later) query rows first when causal.
+// Query tile pair, head and batch entry of a job's work item.  (batch entry, head) pairs are taken in blocks of
+// `hb`; inside a block the pairs come row by row, heavier (later) query rows first when causal, and the heads
+// of one row one after the other.  hb = 1 is head by head.
 struct ItemCoords {
   int pair, h, b;
 };
-__device__ __forceinline__ ItemCoords item_coords(int item, int n_pairs, int Hq, int causal) {
-  const int pidx = item % n_pairs, bh = item / n_pairs;
+__device__ __forceinline__ ItemCoords item_coords(int item, int n_pairs, int hb, int B, int Hq, int causal) {
+  const int blk = item / (hb * n_pairs), rem = item - blk * hb * n_pairs;
+  const int n = min(hb, B * Hq - blk * hb);  // heads of this block
+  const int pidx = rem / n, bh = blk * hb + rem % n;
   return ItemCoords{causal ? n_pairs - 1 - pidx : pidx, bh % Hq, bh / Hq};
 }
 
@@ -104,8 +107,8 @@ attn_fwd_kernel(const __grid_constant__ FwdMaps maps, const __grid_constant__ Fw
     while (jid + 1 < a.njobs && (int)blockIdx.x >= a.job[jid + 1].x_begin) ++jid;
     ctl->jid = jid;
     ctl->job = a.job[jid];
-    // CTAs are dispatched in grid order: job by job, inside a job batch entry by batch entry and head by
-    // head (the CTAs running at one time share a few heads' K/V through L2), heavier query rows first.
+    // CTAs are dispatched in grid order: job by job, inside a job in the order of item_coords (the CTAs
+    // running at one time share a few heads' K/V through L2).
     int local = (int)blockIdx.x - a.job[jid].x_begin;
     ctl->slot = -1;
     ctl->part = 0;
@@ -114,7 +117,7 @@ attn_fwd_kernel(const __grid_constant__ FwdMaps maps, const __grid_constant__ Fw
       ctl->part = ctl->slot % a.nsplit;
       local = a.split_begin + ctl->slot / a.nsplit;
     }
-    const ItemCoords it = item_coords(local, a.job[jid].n_pairs, a.Hq, a.causal);
+    const ItemCoords it = item_coords(local, a.job[jid].n_pairs, a.head_block, a.B, a.Hq, a.causal);
     ctl->pair = it.pair;
     ctl->h = it.h;
     ctl->b = it.b;
@@ -649,7 +652,7 @@ struct FwdMergeArgs {
   long long o_sb, o_ss, o_sh;
   float* lse;
   long long lse_sb, lse_sh;
-  int Sq, Hq, n_pairs, causal, first_item, nsplit;
+  int Sq, B, Hq, n_pairs, head_block, causal, first_item, nsplit;
   float scale, scale_log2;
 };
 
@@ -661,7 +664,7 @@ __global__ void __launch_bounds__(256) fwd_split_merge_kernel(const FwdMergeArgs
   const int lane = threadIdx.x & 31, group = threadIdx.x >> 5;  // column group: 16 columns
   const int item = blockIdx.x;
   const int r = blockIdx.y * 32 + lane;
-  const ItemCoords it = item_coords(a.first_item + item, a.n_pairs, a.Hq, a.causal);
+  const ItemCoords it = item_coords(a.first_item + item, a.n_pairs, a.head_block, a.B, a.Hq, a.causal);
   const int qrow = it.pair * kRows + r;
   if (qrow >= a.Sq) return;
   const long long slot0 = (long long)item * a.nsplit;
@@ -806,6 +809,22 @@ long long attn_fwd_workspace(const mb_attn_fwd_args* x) {
   return plan_split(x).slots * (long long)kSlotBytes;
 }
 
+constexpr long long kL2Bytes = 64ll << 20;
+// Heads whose items are dispatched together, longest first, in a causal launch: as many as have their K/V in kL2Bytes
+// of L2, in equal blocks.  Head by head, the longest items of the last heads start when most of the work is
+// done and the launch waits for them.  Measured (B200): batch 2, 2 999 rows, 16 heads over 4: 107 us head by
+// head, 92 us over all heads; 32 768 rows, 32 heads (16 MiB a head): 16, 32, 64 and 128 MiB alike within 1 %.
+static int causal_head_block(const FwdArgs& a) {
+  long long rows = 0;
+  for (int s = 0; s < a.nseg; ++s) rows += a.seg_sk[s];
+  const long long kv_bytes = max(rows * kD * 4, 1ll);  // K and V of one K/V head
+  const long long heads = (long long)a.B * a.Hq;
+  const long long fit = max(kL2Bytes / kv_bytes, 1ll) * a.group;
+  if (fit >= heads) return (int)heads;
+  const long long blocks = (heads + fit - 1) / fit;
+  return (int)((heads + blocks - 1) / blocks);
+}
+
 static int make_tile_map(CUtensorMap* map, const void* ptr, int D, int H, int S, int B, long long sb, long long ss,
                          long long sh) {
   cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)H, (cuuint64_t)S, (cuuint64_t)B};
@@ -945,6 +964,8 @@ static int launch_fwd(const mb_attn_fwd_multi_args* x, const FwdSplit& split, vo
   a.status = x->status ? x->status : default_status_word();
   if (a.status == nullptr) return MB_E_CUDA;
 
+  a.head_block = 1;
+  if (a.causal && !has_flags && njobs == 1) a.head_block = causal_head_block(a);
   a.split_begin = split.split_begin;
   a.nsplit = split.nsplit;
   if (split.slots > 0) {
@@ -961,7 +982,7 @@ static int launch_fwd(const mb_attn_fwd_multi_args* x, const FwdSplit& split, vo
     m.part_o = a.part_o; m.part_ml = a.part_ml;
     m.o = J.o; m.o_sb = J.o_sb; m.o_ss = J.o_ss; m.o_sh = J.o_sh;
     m.lse = J.lse; m.lse_sb = J.lse_sb; m.lse_sh = J.lse_sh;
-    m.Sq = J.Sq; m.Hq = a.Hq; m.n_pairs = J.n_pairs; m.causal = a.causal;
+    m.Sq = J.Sq; m.B = a.B; m.Hq = a.Hq; m.n_pairs = J.n_pairs; m.head_block = a.head_block; m.causal = a.causal;
     m.first_item = split.split_begin; m.nsplit = split.nsplit;
     m.scale = a.scale; m.scale_log2 = a.scale_log2;
     const int rows = min(2 * kBM, J.Sq);  // a job shorter than one item has no rows past Sq

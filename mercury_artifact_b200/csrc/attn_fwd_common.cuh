@@ -56,6 +56,7 @@ struct FwdArgs {
   FwdJob job[kMaxJobs];
   int njobs;
   int B, Hq, group;
+  int head_block;  // (batch entry, head) pairs dispatched together (see item_coords)
   int nseg;
   int seg_sk[MB_MAX_SEGMENTS];
   int seg_koff[MB_MAX_SEGMENTS];
