@@ -117,9 +117,9 @@ attn_fwd_kernel(const __grid_constant__ FwdMaps maps, const __grid_constant__ Fw
       ctl->part = ctl->slot % a.nsplit;
       local = a.split_begin + ctl->slot / a.nsplit;
     }
-    const ItemCoords it = item_coords(local, a.job[jid].n_pairs, a.head_block, a.B, a.Hq, a.causal);
+    const ItemCoords it = item_coords(local, a.job[jid].n_pairs, a.head_block, a.B, a.Hq >> a.pack_shift, a.causal);
     ctl->pair = it.pair;
-    ctl->h = it.h;
+    ctl->h = it.h << a.pack_shift;
     ctl->b = it.b;
   }
   __syncthreads();
@@ -154,7 +154,7 @@ attn_fwd_kernel(const __grid_constant__ FwdMaps maps, const __grid_constant__ Fw
     if (lane < a.nseg && ((J.seg_mask >> lane) & 1u)) {
 #pragma unroll
       for (int i = 0; i < 2; ++i)
-        n[i] = visible_tiles(q0 + i * kBM, J.Sq, J.q_off, a.causal, a.seg_sk[lane], a.seg_koff[lane]);
+        n[i] = visible_tiles(q0 + i * kBM, J.Sq, a.pack_shift, J.q_off, a.causal, a.seg_sk[lane], a.seg_koff[lane]);
     }
     int lo = 0;
     if (ctl->slot >= 0) {
@@ -209,12 +209,14 @@ attn_fwd_kernel(const __grid_constant__ FwdMaps maps, const __grid_constant__ Fw
         asm volatile("fence.proxy.async;" ::: "memory");
       }
       if (ok) {
-        const int act0 = q0 < J.Sq, act1 = q0 + kBM < J.Sq;
+        const int rows = J.Sq << a.pack_shift;
+        const int act0 = q0 < rows, act1 = q0 + kBM < rows;
         mbar_expect_tx(&ctl->q_full, (act0 + act1) * kTileBytes);
         for (int i = 0; i < 2; ++i) {
-          if (q0 + i * kBM < J.Sq) {
-            tma_load_4d(sQ + i * kTileBytes, qmap, &ctl->q_full, 0, ctl->h, q0 + i * kBM, ctl->b);
-            tma_load_4d(sQ + i * kTileBytes + kHalfBytes, qmap, &ctl->q_full, 64, ctl->h, q0 + i * kBM, ctl->b);
+          if (q0 + i * kBM < rows) {
+            const int r0 = (q0 + i * kBM) >> a.pack_shift;
+            tma_load_4d(sQ + i * kTileBytes, qmap, &ctl->q_full, 0, ctl->h, r0, ctl->b);
+            tma_load_4d(sQ + i * kTileBytes + kHalfBytes, qmap, &ctl->q_full, 64, ctl->h, r0, ctl->b);
           }
         }
       }
@@ -368,14 +370,16 @@ attn_fwd_kernel(const __grid_constant__ FwdMaps maps, const __grid_constant__ Fw
     const uint32_t tS = tmem + lane_field;
     const uint32_t tPi = tmem + 128 + i * 64 + lane_field;
     const uint32_t tOi = tmem + 256 + i * 128 + lane_field;
-    // global position used by the causal rule; the row inside the job's Q is qpos - J.q_off
-    const int qpos = J.q_off + q0 + i * kBM + row;
+    // global position used by the causal rule (of the tile's first row: qfirst); the row inside the job's Q is
+    // qpos - J.q_off
+    const int qfirst = J.q_off + ((q0 + i * kBM) >> a.pack_shift);
+    const int qpos = qfirst + (row >> a.pack_shift);
 
     float m_ref = -INFINITY;  // reference max (raw score units)
     float l = 0.f;            // running sum of exp2
     int cnt = 0;
     bool ok = true;
-    if (J.st_in && q0 + i * kBM < J.Sq) {
+    if (J.st_in && q0 + i * kBM < J.Sq) {  // (carried states go with unpacked rows)
       const int qrow = qpos - J.q_off;  // row inside the job's Q
       const long long st_row = ((long long)ctl->b * a.Hq + ctl->h) * J.Sq + qrow;
       // Continue where an earlier job stopped: its unnormalised rows go back into tensor memory, its
@@ -433,7 +437,7 @@ attn_fwd_kernel(const __grid_constant__ FwdMaps maps, const __grid_constant__ Fw
         // masking: only tiles that cross the segment end or the causal diagonal
         const int k0 = jt * kBN;
         const bool tile_needs_mask =
-            (k0 + kBN > sk) || (a.causal && (koff + k0 + kBN - 1 > qpos - row));  // qpos - row: the tile's first row
+            (k0 + kBN > sk) || (a.causal && (koff + k0 + kBN - 1 > qfirst));
         if (tile_needs_mask) {
           int limit = sk - k0;  // columns >= limit are invisible
           if (a.causal) limit = min(limit, qpos - koff - k0 + 1);
@@ -528,7 +532,7 @@ attn_fwd_kernel(const __grid_constant__ FwdMaps maps, const __grid_constant__ Fw
     // epilogue.  Final job: O / l -> bf16, LSE = ln(sum exp(scale * s)).  Job that hands its state on:
     // the unnormalised rows, the maximum and the sum, as they are.  Tiles whose rows all lie past Sq skip it.
     const int qrow = qpos - J.q_off;  // row inside the job's Q
-    if (ok && qrow - row < J.Sq) {
+    if (ok && qfirst - J.q_off < J.Sq) {
       const long long st_row = ((long long)ctl->b * a.Hq + ctl->h) * J.Sq + qrow;
       const bool have_acc = cnt > 0 || J.st_in;   // tensor memory holds this tile's rows
       if (cnt > 0) ok = mbar_wait_warp(&ctl->o_full[i], (cnt - 1) & 1, abort_word, MB_ERR_TIMEOUT_O, a.wait_cycles);
@@ -575,7 +579,8 @@ attn_fwd_kernel(const __grid_constant__ FwdMaps maps, const __grid_constant__ Fw
           if (store) *reinterpret_cast<float2*>(J.st_ml + st_row * 2) = make_float2(m_ref, l);
         } else {
           const float inv_l = (have_acc && l > 0.f) ? 1.f / l : 0.f;
-          __nv_bfloat16* optr = J.o + (long long)ctl->b * J.o_sb + (long long)qrow * J.o_ss + (long long)ctl->h * J.o_sh;
+          const int head = ctl->h + (row & ((1 << a.pack_shift) - 1));
+          __nv_bfloat16* optr = J.o + (long long)ctl->b * J.o_sb + (long long)qrow * J.o_ss + (long long)head * J.o_sh;
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
             uint32_t orow[32];
@@ -601,7 +606,7 @@ attn_fwd_kernel(const __grid_constant__ FwdMaps maps, const __grid_constant__ Fw
           }
           if (store) {
             const float lse = (have_acc && l > 0.f) ? (m_ref * a.scale + __logf(l)) : -INFINITY;
-            J.lse[(long long)ctl->b * J.lse_sb + (long long)ctl->h * J.lse_sh + qrow] = lse;
+            J.lse[(long long)ctl->b * J.lse_sb + (long long)head * J.lse_sh + qrow] = lse;
           }
         }
       }
@@ -652,7 +657,7 @@ struct FwdMergeArgs {
   long long o_sb, o_ss, o_sh;
   float* lse;
   long long lse_sb, lse_sh;
-  int Sq, B, Hq, n_pairs, head_block, causal, first_item, nsplit;
+  int Sq, B, Hq, n_pairs, pack_shift, head_block, causal, first_item, nsplit;
   float scale, scale_log2;
 };
 
@@ -664,8 +669,9 @@ __global__ void __launch_bounds__(256) fwd_split_merge_kernel(const FwdMergeArgs
   const int lane = threadIdx.x & 31, group = threadIdx.x >> 5;  // column group: 16 columns
   const int item = blockIdx.x;
   const int r = blockIdx.y * 32 + lane;
-  const ItemCoords it = item_coords(a.first_item + item, a.n_pairs, a.head_block, a.B, a.Hq, a.causal);
-  const int qrow = it.pair * kRows + r;
+  const ItemCoords it = item_coords(a.first_item + item, a.n_pairs, a.head_block, a.B, a.Hq >> a.pack_shift, a.causal);
+  const int prow = it.pair * kRows + r;  // row over (query, head of the group)
+  const int qrow = prow >> a.pack_shift, head = (it.h << a.pack_shift) + (prow & ((1 << a.pack_shift) - 1));
   if (qrow >= a.Sq) return;
   const long long slot0 = (long long)item * a.nsplit;
   const float2* ml = a.part_ml + slot0 * kRows + r;
@@ -696,7 +702,7 @@ __global__ void __launch_bounds__(256) fwd_split_merge_kernel(const FwdMergeArgs
     }
   }
   const float inv = l > 0.f ? 1.f / l : 0.f;
-  uint4* dst = reinterpret_cast<uint4*>(a.o + it.b * a.o_sb + qrow * a.o_ss + it.h * a.o_sh + group * 16);
+  uint4* dst = reinterpret_cast<uint4*>(a.o + it.b * a.o_sb + qrow * a.o_ss + head * a.o_sh + group * 16);
 #pragma unroll
   for (int v = 0; v < 2; ++v) {
     uint4 w;
@@ -706,7 +712,7 @@ __global__ void __launch_bounds__(256) fwd_split_merge_kernel(const FwdMergeArgs
     w.w = pack_bf16x2(acc[v * 8 + 6] * inv, acc[v * 8 + 7] * inv);
     dst[v] = w;
   }
-  if (group == 0) a.lse[it.b * a.lse_sb + it.h * a.lse_sh + qrow] = l > 0.f ? m * a.scale + __logf(l) : -INFINITY;
+  if (group == 0) a.lse[it.b * a.lse_sb + head * a.lse_sh + qrow] = l > 0.f ? m * a.scale + __logf(l) : -INFINITY;
 }
 
 // ---------------------------------------------------------------------------
@@ -734,11 +740,28 @@ static int sm_count() {
 // others idle.  Measured (B200): 100 queries against 16 384 keys, 32 heads over 8 K/V heads, 164 us whole, 55 us in
 // 4 shares; 4 096 queries against 32 768 keys, 32 heads (3.46 waves), 1.89 ms whole, 1.76 ms with the last
 // 68 items in 2 shares.  The price of a split is one CTA start per share and one launch that merges.
+// log2 of the query heads that share a tile row by row (row = query * heads + head).  The heads of a group read the
+// same K/V, so a tile of 128 rows may hold all of them for 128 / group queries instead of one of them for 128:
+// worth it when the queries of one head leave much of a pair of tiles empty, which is where it saves an eighth of the
+// pairs.  Grouped layouts only, groups that divide a tile.  Measured (B200): 100 queries against 16 384 keys, 32
+// heads over 8: 55 us head by head (32 pairs, half empty), 42 us packed (16 pairs).
+static int plan_pack(int sq, int hq, int hkv) {
+  if (hkv <= 0 || hq % hkv != 0) return 0;
+  const int group = hq / hkv;
+  int shift = 0;
+  while ((1 << shift) < group && shift < 8) ++shift;
+  if ((1 << shift) != group || group > kBM || sq > INT_MAX / group - 2 * kBM) return 0;
+  const long long apart = (long long)group * ((sq + 2ll * kBM - 1) / (2 * kBM));  // pairs of a group, head by head
+  const long long packed = ((long long)sq * group + 2 * kBM - 1) / (2 * kBM);
+  return packed * 8 <= apart * 7 ? shift : 0;
+}
+
 static FwdSplit plan_split(const mb_attn_fwd_args* x) {
   const FwdSplit whole{INT_MAX, 1, 0};
   if (x->sq <= 0 || x->softmax_scale <= 0.f) return whole;
   const int sms = sm_count();
-  const int np = (x->sq + 2 * kBM - 1) / (2 * kBM), heads = x->hq;
+  const int pack_shift = plan_pack(x->sq, x->hq, x->hkv);
+  const int np = ((x->sq << pack_shift) + 2 * kBM - 1) / (2 * kBM), heads = x->hq >> pack_shift;
   const long long items = (long long)np * heads * x->batch;
   if (sms <= 0 || items > INT_MAX) return whole;
   // A launch over several shards is cut in its last wave only: smaller ones add up in the order of the chained
@@ -755,7 +778,7 @@ static FwdSplit plan_split(const mb_attn_fwd_args* x) {
     t_max = 0;
     for (int p = 0; p < np; ++p) {
       long long t = 0;
-      const long long last = (long long)x->q_off + min((p + 1) * 2 * kBM - 1, x->sq - 1);
+      const long long last = (long long)x->q_off + min(((p + 1) * 2 * kBM - 1) >> pack_shift, x->sq - 1);
       for (int s = 0; s < x->nseg; ++s) {
         const long long vis = min((long long)x->seg[s].sk, last - x->seg[s].k_off + 1);
         if (vis > 0) t += (vis + kBN - 1) / kBN;
@@ -818,18 +841,18 @@ static int causal_head_block(const FwdArgs& a) {
   long long rows = 0;
   for (int s = 0; s < a.nseg; ++s) rows += a.seg_sk[s];
   const long long kv_bytes = max(rows * kD * 4, 1ll);  // K and V of one K/V head
-  const long long heads = (long long)a.B * a.Hq;
-  const long long fit = max(kL2Bytes / kv_bytes, 1ll) * a.group;
+  const long long heads = (long long)a.B * (a.Hq >> a.pack_shift);
+  const long long fit = max(kL2Bytes / kv_bytes, 1ll) * (a.group >> a.pack_shift);
   if (fit >= heads) return (int)heads;
   const long long blocks = (heads + fit - 1) / fit;
   return (int)((heads + blocks - 1) / blocks);
 }
 
 static int make_tile_map(CUtensorMap* map, const void* ptr, int D, int H, int S, int B, long long sb, long long ss,
-                         long long sh) {
+                         long long sh, int pack_shift = 0) {
   cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)H, (cuuint64_t)S, (cuuint64_t)B};
   cuuint64_t strides[3] = {(cuuint64_t)sh * 2, (cuuint64_t)ss * 2, (cuuint64_t)sb * 2};
-  cuuint32_t box[4] = {64, 1, (cuuint32_t)kBN, 1};
+  cuuint32_t box[4] = {64, 1u << pack_shift, (cuuint32_t)kBN >> pack_shift, 1};  // 128 rows, heads innermost
   cuuint32_t estr[4] = {1, 1, 1, 1};
   return encode_tiled_bf16(map, const_cast<void*>(ptr), 4, dims, strides, box, estr);
 }
@@ -842,7 +865,9 @@ void set_peer_wait_ms(unsigned ms) { g_peer_wait_ms = ms == 0 ? 1 : ms; }
 // 2e6 cycles per millisecond is at least the requested time.
 long long peer_wait_cycles() { return g_peer_wait_ms * 2000000LL; }
 
-static int launch_fwd(const mb_attn_fwd_multi_args* x, const FwdSplit& split, void* ws, cudaStream_t stream) {
+// pack_shift != 0: one job without carried state or chain (see plan_pack).
+static int launch_fwd(const mb_attn_fwd_multi_args* x, int pack_shift, const FwdSplit& split, void* ws,
+                      cudaStream_t stream) {
   if (x == nullptr) return MB_E_INVALID;
   if (x->head_dim != kD) return MB_E_UNSUPPORTED;
   if (x->batch <= 0 || x->hq <= 0 || x->hkv <= 0 || x->hq % x->hkv != 0) return MB_E_INVALID;
@@ -909,7 +934,8 @@ static int launch_fwd(const mb_attn_fwd_multi_args* x, const FwdSplit& split, vo
     }
     if (qmap < 0) {
       if (nqmaps == kMaxQMaps) return MB_E_INVALID;
-      if (make_tile_map(&maps.q[nqmaps], g.q, kD, x->hq, g.sq, x->batch, g.q_stride_b, g.q_stride_s, g.q_stride_h))
+      if (make_tile_map(&maps.q[nqmaps], g.q, kD, x->hq, g.sq, x->batch, g.q_stride_b, g.q_stride_s, g.q_stride_h,
+                        pack_shift))
         return MB_E_TENSORMAP;
       qmap_of[nqmaps] = &g;
       qmap = nqmaps++;
@@ -930,13 +956,13 @@ static int launch_fwd(const mb_attn_fwd_multi_args* x, const FwdSplit& split, vo
       if (seg_new[s] >= 0 && (g.seg_mask == 0 || ((g.seg_mask >> s) & 1u))) mask |= 1u << seg_new[s];
     J.seg_mask = mask;
     J.x_begin = x_total;
-    J.n_pairs = (g.sq + 2 * kBM - 1) / (2 * kBM);
+    J.n_pairs = ((g.sq << pack_shift) + 2 * kBM - 1) / (2 * kBM);
     J.q_flag = g.q_ready_flag;
     J.q_flag_value = g.q_ready_value;
     J.done_flag = g.done_flag;
     J.done_value = g.done_value;
     J.done_counter = g.done_counter;
-    J.n_ctas = J.n_pairs * x->hq * x->batch;
+    J.n_ctas = J.n_pairs * (x->hq >> pack_shift) * x->batch;
     J.st_o = g.state_o;
     J.st_ml = g.state_ml;
     J.st_in = g.state_in ? 1 : 0;
@@ -964,6 +990,7 @@ static int launch_fwd(const mb_attn_fwd_multi_args* x, const FwdSplit& split, vo
   a.status = x->status ? x->status : default_status_word();
   if (a.status == nullptr) return MB_E_CUDA;
 
+  a.pack_shift = pack_shift;
   a.head_block = 1;
   if (a.causal && !has_flags && njobs == 1) a.head_block = causal_head_block(a);
   a.split_begin = split.split_begin;
@@ -982,10 +1009,11 @@ static int launch_fwd(const mb_attn_fwd_multi_args* x, const FwdSplit& split, vo
     m.part_o = a.part_o; m.part_ml = a.part_ml;
     m.o = J.o; m.o_sb = J.o_sb; m.o_ss = J.o_ss; m.o_sh = J.o_sh;
     m.lse = J.lse; m.lse_sb = J.lse_sb; m.lse_sh = J.lse_sh;
-    m.Sq = J.Sq; m.B = a.B; m.Hq = a.Hq; m.n_pairs = J.n_pairs; m.head_block = a.head_block; m.causal = a.causal;
+    m.Sq = J.Sq; m.B = a.B; m.Hq = a.Hq; m.n_pairs = J.n_pairs;
+    m.pack_shift = a.pack_shift; m.head_block = a.head_block; m.causal = a.causal;
     m.first_item = split.split_begin; m.nsplit = split.nsplit;
     m.scale = a.scale; m.scale_log2 = a.scale_log2;
-    const int rows = min(2 * kBM, J.Sq);  // a job shorter than one item has no rows past Sq
+    const int rows = min(2 * kBM, J.Sq << a.pack_shift);  // a job shorter than one item has no rows past Sq
     fwd_split_merge_kernel<<<dim3(split.slots / split.nsplit, (rows + 31) / 32), 256, 0, stream>>>(m);
     if (!cuda_ok(cudaGetLastError(), "launch fwd_split_merge_kernel")) return MB_E_CUDA;
   }
@@ -993,7 +1021,7 @@ static int launch_fwd(const mb_attn_fwd_multi_args* x, const FwdSplit& split, vo
 }
 
 int launch_attn_fwd_multi(const mb_attn_fwd_multi_args* x, cudaStream_t stream) {
-  return launch_fwd(x, FwdSplit{INT_MAX, 1, 0}, nullptr, stream);
+  return launch_fwd(x, 0, FwdSplit{INT_MAX, 1, 0}, nullptr, stream);
 }
 
 // One query shard: the single-job form of the launch above.  With a workspace of attn_fwd_workspace(x) bytes the
@@ -1025,7 +1053,7 @@ int launch_attn_fwd(const mb_attn_fwd_args* x, void* ws, unsigned long long ws_b
     if (split.slots * (unsigned long long)kSlotBytes > ws_bytes || (reinterpret_cast<uintptr_t>(ws) & 15u))
       split = FwdSplit{INT_MAX, 1, 0};
   }
-  return launch_fwd(&m, split, ws, stream);
+  return launch_fwd(&m, plan_pack(x->sq, x->hq, x->hkv), split, ws, stream);
 }
 
 }  // namespace mb

@@ -56,6 +56,7 @@ struct FwdArgs {
   FwdJob job[kMaxJobs];
   int njobs;
   int B, Hq, group;
+  int pack_shift;  // log2 of the heads whose rows share a tile (0: a tile holds rows of one head)
   int head_block;  // (batch entry, head) pairs dispatched together (see item_coords)
   int nseg;
   int seg_sk[MB_MAX_SEGMENTS];
@@ -102,12 +103,12 @@ constexpr int kFwdSmemBytes = 2 * kTileBytes + kFwdStages * kTileBytes + 1024 /*
 static_assert(sizeof(FwdSmem) <= 1024, "control block too large");
 static_assert(kFwdSmemBytes <= 232448, "shared memory budget of one CTA");
 
-// Number of K/V tiles of a segment that a query tile starting at row q0 can see.
-__device__ __forceinline__ int visible_tiles(int q0, int Sq, int q_off, int causal, int sk, int koff) {
-  if (q0 >= Sq || sk <= 0) return 0;
+// Number of K/V tiles of a segment that a query tile starting at (packed) row q0 can see.
+__device__ __forceinline__ int visible_tiles(int q0, int Sq, int pack_shift, int q_off, int causal, int sk, int koff) {
+  if (q0 >> pack_shift >= Sq || sk <= 0) return 0;
   int nt = (sk + kBN - 1) / kBN;
   if (causal) {
-    int last_row = min(q0 + kBM - 1, Sq - 1);
+    int last_row = min((q0 + kBM - 1) >> pack_shift, Sq - 1);
     long long max_k = (long long)q_off + last_row - koff;  // largest visible local key index
     if (max_k < 0) return 0;
     long long lim = max_k / kBN + 1;

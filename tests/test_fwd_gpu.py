@@ -390,6 +390,7 @@ SPLIT_CASES = [
     (1, 1300, 900, 2, 2, True, -300, 1, True),    # rows without any visible key in every share
     (1, 33, 1500, 6, 2, False, 0, 1, True),       # a group that does not divide a tile: heads apart
     (1, 65, 300, 128, 1, True, 235, 1, False),    # the largest group that fits a tile; too few keys to split
+    (1, 65, 900, 128, 1, True, 835, 1, True),     # the same with enough
     (3, 6390, 1400, 2, 2, False, 0, 1, True),     # 150 items: the last two split, the first 148 whole
     (3, 6390, 1400, 2, 2, False, 0, 3, True),     # the same over three shards
     (2, 300, 1400, 4, 2, True, 1100, 3, False),   # several shards, less than a wave: whole
