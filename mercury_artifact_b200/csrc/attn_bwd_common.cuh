@@ -51,7 +51,22 @@ struct BwdArgs {
   long long o_sb, o_ss, o_sh;
   int out_mode;  // 0 bf16 store, 1 fp32 store, 2 fp32 accumulate
   int* status;
+  // order of the owner tiles in the (one-dimensional) grid, see own_coords
+  int n_own, n_heads, head_block, own_last_first;
 };
+
+// Owner tile, head and batch entry of a CTA.  (batch entry, head) pairs are taken in blocks of head_block; inside a
+// block the tiles come one after the other, the ones with the most steps first when causal, and the heads of
+// one tile position one after the other.  head_block = 1 is head by head.
+struct OwnCoords {
+  int tile, h, b;
+};
+__device__ __forceinline__ OwnCoords own_coords(const BwdArgs& a, int item) {
+  const int blk = item / (a.head_block * a.n_own), rem = item - blk * a.head_block * a.n_own;
+  const int n = min(a.head_block, a.B * a.n_heads - blk * a.head_block);  // heads of this block
+  const int t = rem / n, bh = blk * a.head_block + rem % n;
+  return OwnCoords{a.own_last_first ? a.n_own - 1 - t : t, bh % a.n_heads, bh / a.n_heads};
+}
 
 struct BwdSmem {
   uint64_t own_full;
@@ -222,6 +237,6 @@ __device__ __forceinline__ void ew_compute(const uint32_t (&xr)[32], const uint3
 }
 
 // single-pass kernel (attn_bwd_fused.cu), launched by launch_attn_bwd for MB_BWD_MODE_FUSED
-int launch_attn_bwd_fused(const BwdMaps& maps, const BwdArgs& a, dim3 grid, cudaStream_t stream);
+int launch_attn_bwd_fused(const BwdMaps& maps, const BwdArgs& a, int n_ctas, cudaStream_t stream);
 
 }  // namespace mb

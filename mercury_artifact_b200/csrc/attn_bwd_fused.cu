@@ -71,6 +71,7 @@ constexpr int kFusedSmemBytes =
 static_assert(kFusedSmemBytes <= 232448, "shared memory budget of one CTA");
 
 struct FusedSmem {
+  OwnCoords own;  // what this CTA owns: read where it is needed, so that it holds no registers across the loops
   uint64_t own_full;
   uint64_t str_full[kFusedStages];
   uint64_t str_empty[kFusedStages];
@@ -138,11 +139,7 @@ __global__ void __maxnreg__(kLaunchRegs) attn_bwd_fused_kernel(const __grid_cons
   static_assert((kFusedStages * kBwdStageBytes) % 1024 == 0, "dS^T tile must stay 1024-byte aligned");
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int own0 = blockIdx.x * kOwnRows;
-  const int h_own = blockIdx.y;  // K/V head
-  const int b = blockIdx.z;
   const int n_sub = a.group;     // query heads streamed per segment
-  const int h_str_base = h_own * a.group;
 
   if (tid == 0) {
     mbar_init(&ctl->own_full, 1);
@@ -166,7 +163,9 @@ __global__ void __maxnreg__(kLaunchRegs) attn_bwd_fused_kernel(const __grid_cons
   }
   if (tid < MB_MAX_SEGMENTS) {  // one thread per segment: its range of 64-row steps for this owner tile
     int f = 0, l = 0;
-    if (tid < a.nseg) step_range(a, own0, tid, &f, &l);
+    const OwnCoords own = own_coords(a, blockIdx.x);
+    if (tid == 0) ctl->own = own;
+    if (tid < a.nseg) step_range(a, own.tile * kOwnRows, tid, &f, &l);
     ctl->seg_first[tid] = f;
     ctl->seg_last[tid] = l;
   }
@@ -190,6 +189,7 @@ __global__ void __maxnreg__(kLaunchRegs) attn_bwd_fused_kernel(const __grid_cons
     // ------------------------------------------------------------------ loader
     fused_regs_aux<kLaunchRegs>();
     if (lane == 0 && total_steps > 0) {
+      const int own0 = ctl->own.tile * kOwnRows, h_own = ctl->own.h, b = ctl->own.b;
       mbar_expect_tx(&ctl->own_full, 2 * kOwnTileBytes);
       tma_load_4d(sOwn, &maps.own, &ctl->own_full, 0, h_own, own0, b);
       tma_load_4d(sOwn + kOwnHalfBytes, &maps.own, &ctl->own_full, 64, h_own, own0, b);
@@ -205,7 +205,7 @@ __global__ void __maxnreg__(kLaunchRegs) attn_bwd_fused_kernel(const __grid_cons
           asm volatile("fence.proxy.async;" ::: "memory");
         }
         for (int g = 0; g < n_sub && ok; ++g) {
-          const int h_str = h_str_base + g;
+          const int h_str = h_own * a.group + g;
           for (int t = f; t < l; ++t) {
             const int stage = n % kFusedStages, round = n / kFusedStages;
             if (round > 0 && !mbar_wait(&ctl->str_empty[stage], (round - 1) & 1, abort_word, MB_ERR_TIMEOUT_KV_EMPTY,
@@ -343,7 +343,8 @@ __global__ void __maxnreg__(kLaunchRegs) attn_bwd_fused_kernel(const __grid_cons
       const int f = ctl->seg_first[s], l = ctl->seg_last[s];
       const int rows = a.seg_rows[s];
       for (int g = 0; g < n_sub && ok; ++g) {
-        float* acc_base = a.seg_dq[s] + ((long long)b * a.Hq + (h_str_base + g)) * a.seg_stat_pad[s] * kBD;
+        float* acc_base =
+            a.seg_dq[s] + ((long long)ctl->own.b * a.Hq + (ctl->own.h * a.group + g)) * a.seg_stat_pad[s] * kBD;
         for (int st = f; st < l; ++st, ++t) {
           ok = mbar_wait_warp(&ctl->dq_full[t & 1], (t >> 1) & 1, abort_word, MB_ERR_TIMEOUT_O, a.wait_cycles);
           {
@@ -403,7 +404,7 @@ __global__ void __maxnreg__(kLaunchRegs) attn_bwd_fused_kernel(const __grid_cons
     const int quarter = warp & 3, half = warp >> 2;
     const int row = (quarter << 5) | lane;  // key row == tensor-memory lane
     const uint32_t lane_field = static_cast<uint32_t>(quarter << 5) << 16;
-    const int own_pos = a.own_off + own0 + row;
+    const int own_pos = a.own_off + ctl->own.tile * kOwnRows + row;
     // my row of the dS^T tile in shared memory: four 16-byte chunks (32 queries), 128-byte swizzle
     const int swz = row & 7;
     bool ok = true;
@@ -463,6 +464,7 @@ __global__ void __maxnreg__(kLaunchRegs) attn_bwd_fused_kernel(const __grid_cons
     }
 
     // epilogue: each warp stores its lane quarter x column half of dK and dV
+    const int own0 = ctl->own.tile * kOwnRows;
     if (ok && own0 < a.own_rows) {
       const bool have = total_steps > 0;
       if (have) ok = mbar_wait_warp(&ctl->acc_full, 0, abort_word, MB_ERR_TIMEOUT_O, a.wait_cycles);
@@ -472,7 +474,7 @@ __global__ void __maxnreg__(kLaunchRegs) attn_bwd_fused_kernel(const __grid_cons
         for (int which = 0; which < 2; ++which) {
           void* base = which ? a.out2 : a.out1;
           const float mul = which ? 1.f : a.scale;  // dK carries the softmax scale, dV does not
-          const long long off = (long long)b * a.o_sb + (long long)(own0 + row) * a.o_ss + (long long)h_own * a.o_sh;
+          const long long off = (long long)ctl->own.b * a.o_sb + (long long)(own0 + row) * a.o_ss + (long long)ctl->own.h * a.o_sh;
 #pragma unroll
           for (int c = 0; c < 2; ++c) {
             uint32_t acc[32];
@@ -557,7 +559,7 @@ __global__ void __launch_bounds__(256) dq_convert_kernel(const DqConvertArgs a) 
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
-int launch_attn_bwd_fused(const BwdMaps& maps, const BwdArgs& a, dim3 grid, cudaStream_t stream) {
+int launch_attn_bwd_fused(const BwdMaps& maps, const BwdArgs& a, int n_ctas, cudaStream_t stream) {
   static bool done[64] = {};
   int dev = 0;
   if (!cuda_ok(cudaGetDevice(&dev), "cudaGetDevice")) return MB_E_CUDA;
@@ -574,8 +576,8 @@ int launch_attn_bwd_fused(const BwdMaps& maps, const BwdArgs& a, dim3 grid, cuda
   // arrival flags are raised by one-warp kernels of the transfer stream: leave them room on every SM
   bool has_flags = false;
   for (int s = 0; s < a.nseg; ++s) has_flags |= a.seg_flag[s] != nullptr;
-  if (has_flags) attn_bwd_fused_kernel<120><<<grid, kFusedThreads, kFusedSmemBytes, stream>>>(maps, a);
-  else attn_bwd_fused_kernel<128><<<grid, kFusedThreads, kFusedSmemBytes, stream>>>(maps, a);
+  if (has_flags) attn_bwd_fused_kernel<120><<<n_ctas, kFusedThreads, kFusedSmemBytes, stream>>>(maps, a);
+  else attn_bwd_fused_kernel<128><<<n_ctas, kFusedThreads, kFusedSmemBytes, stream>>>(maps, a);
   return cuda_ok(cudaGetLastError(), "launch attn_bwd_fused_kernel") ? MB_SUCCESS : MB_E_CUDA;
 }
 
