@@ -661,58 +661,47 @@ struct FwdMergeArgs {
   float scale, scale_log2;
 };
 
-// o = sum_p w_p O_p / sum_p w_p l_p with w_p = exp(scale * (m_p - max m)), in fp32.  A warp handles 32 rows and
-// 16 of the 128 columns, so every load of a share is 512 contiguous bytes; a thread's 16 bf16 results are one
-// 32-byte sector.  Latency-bound: the shares are in L2, and a launch has at most a few blocks per SM.
+// o = sum_p w_p O_p / sum_p w_p l_p with w_p = exp(scale * (m_p - max m)), in fp32.  A block handles 8 rows: warp w
+// columns [16 w, 16 w + 16), a lane 4 columns of one row, so that the lanes of a column group read 128 contiguous
+// bytes of a share and a row's 16 bf16 results are one 32-byte sector.  Latency-bound (the shares are in L2), hence
+// many small blocks and few registers.  Launched with programmatic serialization: blocks come in as those of the
+// attention kernel leave, and wait for its end at griddepcontrol.wait.
+constexpr int kMergeRows = 8;
 __global__ void __launch_bounds__(256) fwd_split_merge_kernel(const FwdMergeArgs a) {
   constexpr int kRows = 2 * kBM;
-  const int lane = threadIdx.x & 31, group = threadIdx.x >> 5;  // column group: 16 columns
+  const int lane = threadIdx.x & 31, chunk = (threadIdx.x >> 5) * 4 + (lane >> 3);  // group of 4 columns
   const int item = blockIdx.x;
-  const int r = blockIdx.y * 32 + lane;
+  const int r = blockIdx.y * kMergeRows + (lane & 7);
   const ItemCoords it = item_coords(a.first_item + item, a.n_pairs, a.head_block, a.B, a.Hq >> a.pack_shift, a.causal);
   const int prow = it.pair * kRows + r;  // row over (query, head of the group)
   const int qrow = prow >> a.pack_shift, head = (it.h << a.pack_shift) + (prow & ((1 << a.pack_shift) - 1));
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   if (qrow >= a.Sq) return;
   const long long slot0 = (long long)item * a.nsplit;
   const float2* ml = a.part_ml + slot0 * kRows + r;
   float m = -INFINITY;
-#pragma unroll 4
+#pragma unroll 8
   for (int p = 0; p < a.nsplit; ++p) m = fmaxf(m, ml[p * kRows].x);
-  float l = 0.f;
-  float acc[16];
-#pragma unroll
-  for (int e = 0; e < 16; ++e) acc[e] = 0.f;
-  const float4* src = a.part_o + (slot0 * 32 + group * 4) * kRows + r;
-#pragma unroll 4
+  float l = 0.f, acc[4] = {0.f, 0.f, 0.f, 0.f};
+  const float4* src = a.part_o + (slot0 * 32 + chunk) * kRows + r;
+#pragma unroll 8
   for (int p = 0; p < a.nsplit; ++p) {
     const float2 s = ml[p * kRows];
     const bool has = !(s.y == 0.f);  // a share without visible keys has stored no rows
-    float4 x[4];
-#pragma unroll
-    for (int v = 0; v < 4; ++v)
-      x[v] = has ? src[((long long)p * 32 + v) * kRows] : make_float4(0.f, 0.f, 0.f, 0.f);
+    const float4 x = has ? src[(long long)p * 32 * kRows] : make_float4(0.f, 0.f, 0.f, 0.f);
     const float w = has ? fast_exp2((s.x - m) * a.scale_log2) : 0.f;
     l = fmaf(w, s.y, l);
-#pragma unroll
-    for (int v = 0; v < 4; ++v) {
-      acc[v * 4 + 0] = fmaf(w, x[v].x, acc[v * 4 + 0]);
-      acc[v * 4 + 1] = fmaf(w, x[v].y, acc[v * 4 + 1]);
-      acc[v * 4 + 2] = fmaf(w, x[v].z, acc[v * 4 + 2]);
-      acc[v * 4 + 3] = fmaf(w, x[v].w, acc[v * 4 + 3]);
-    }
+    acc[0] = fmaf(w, x.x, acc[0]);
+    acc[1] = fmaf(w, x.y, acc[1]);
+    acc[2] = fmaf(w, x.z, acc[2]);
+    acc[3] = fmaf(w, x.w, acc[3]);
   }
   const float inv = l > 0.f ? 1.f / l : 0.f;
-  uint4* dst = reinterpret_cast<uint4*>(a.o + it.b * a.o_sb + qrow * a.o_ss + head * a.o_sh + group * 16);
-#pragma unroll
-  for (int v = 0; v < 2; ++v) {
-    uint4 w;
-    w.x = pack_bf16x2(acc[v * 8 + 0] * inv, acc[v * 8 + 1] * inv);
-    w.y = pack_bf16x2(acc[v * 8 + 2] * inv, acc[v * 8 + 3] * inv);
-    w.z = pack_bf16x2(acc[v * 8 + 4] * inv, acc[v * 8 + 5] * inv);
-    w.w = pack_bf16x2(acc[v * 8 + 6] * inv, acc[v * 8 + 7] * inv);
-    dst[v] = w;
-  }
-  if (group == 0) a.lse[it.b * a.lse_sb + head * a.lse_sh + qrow] = l > 0.f ? m * a.scale + __logf(l) : -INFINITY;
+  uint2 o;
+  o.x = pack_bf16x2(acc[0] * inv, acc[1] * inv);
+  o.y = pack_bf16x2(acc[2] * inv, acc[3] * inv);
+  *reinterpret_cast<uint2*>(a.o + it.b * a.o_sb + qrow * a.o_ss + head * a.o_sh + chunk * 4) = o;
+  if (chunk == 0) a.lse[it.b * a.lse_sb + head * a.lse_sh + qrow] = l > 0.f ? m * a.scale + __logf(l) : -INFINITY;
 }
 
 // ---------------------------------------------------------------------------
@@ -737,9 +726,11 @@ static int sm_count() {
 }
 
 // Without a split a launch of few items runs on as many SMs as it has items, and a last wave of few items leaves the
-// others idle.  Measured (B200): 100 queries against 16 384 keys, 32 heads over 8 K/V heads, 164 us whole, 55 us in
-// 4 shares; 4 096 queries against 32 768 keys, 32 heads (3.46 waves), 1.89 ms whole, 1.76 ms with the last
-// 68 items in 2 shares.  The price of a split is one CTA start per share and one launch that merges.
+// others idle.  Measured (B200), whole / split: 128 queries against 2 048 keys, 8 heads, 27 / 17 us; against 32 768 keys,
+// 315 / 41 us; 1 024 causal rows, 8 heads, 21 / 19 us; 4 096 queries against 32 768 keys, 32 heads (3.46 waves),
+// 1.92 / 1.80 ms with the last 68 items in 2 shares; 5 000 x 5 000, 16 heads, 234 / 188 us.  Shapes that the
+// costs below leave whole, and what a split did to them: 768 x 768, 8 heads, in 6 shares 19 -> 21 us; 2 048 x 4 096, 32
+// heads (108 items in the last wave), in 4 shares 132 -> 145 us.
 // log2 of the query heads that share a tile row by row (row = query * heads + head).  The heads of a group read the
 // same K/V, so a tile of 128 rows may hold all of them for 128 / group queries instead of one of them for 128:
 // worth it when the queries of one head leave much of a pair of tiles empty, which is where it saves an eighth of the
@@ -788,10 +779,12 @@ static FwdSplit plan_split(const mb_attn_fwd_args* x) {
       t_sum += t;
     }
   }
-  // Costs in steps of one K/V tile against both query tiles (about 1.6 us): starting and ending a CTA, and
-  // the extra launch that merges the shares.
-  constexpr double kCta = 2.0, kMerge = 3.0;
+  // Costs in steps of one K/V tile against both query tiles (1.7 us): starting and ending a CTA, the extra launch
+  // that merges the shares, and per share its way through memory.  A wave that leaves SMs idle is also faster
+  // per step (the chip clocks higher): 0.8 of a full one where 68 of 148 SMs work.
+  constexpr double kCta = 1.25, kMerge = 2.0, kSlot = 0.02;
   constexpr int kMaxSplit = 32;
+  auto pace = [&](double busy) { return 0.65 + 0.35 * busy / sms; };
   const long long slot_cap = 3ll * sms;
   FwdSplit best = whole;
   if (x->causal) {
@@ -805,7 +798,7 @@ static FwdSplit plan_split(const mb_attn_fwd_args* x) {
     };
     double t_best = cost(1);
     for (int ns = 2; ns <= kMaxSplit && ns <= t_max && items * ns <= slot_cap; ++ns) {
-      const double t = cost(ns) + kMerge;
+      const double t = cost(ns) + kMerge + kSlot * items * ns;
       if (t < t_best) {
         t_best = t;
         best = FwdSplit{0, ns, (int)(items * ns)};
@@ -814,10 +807,10 @@ static FwdSplit plan_split(const mb_attn_fwd_args* x) {
   } else {
     // Equal items: whole waves run as they are, the items of the last, partly filled one are split.
     const int rest = (int)(items % sms);
-    double t_best = t_max + kCta;
+    double t_best = t_max * pace(rest) + kCta;
     for (int ns = 2; rest > 0 && ns <= kMaxSplit && ns <= t_max && (long long)rest * ns <= slot_cap; ++ns) {
       const int waves = (rest * ns + sms - 1) / sms;
-      const double t = waves * ((double)((t_max + ns - 1) / ns) + kCta) + kMerge;
+      const double t = waves * ((t_max + ns - 1) / ns * pace((double)rest * ns / waves) + kCta) + kMerge + kSlot * rest * ns;
       if (t < t_best) {
         t_best = t;
         best = FwdSplit{(int)(items - rest), ns, rest * ns};
@@ -1014,8 +1007,16 @@ static int launch_fwd(const mb_attn_fwd_multi_args* x, int pack_shift, const Fwd
     m.first_item = split.split_begin; m.nsplit = split.nsplit;
     m.scale = a.scale; m.scale_log2 = a.scale_log2;
     const int rows = min(2 * kBM, J.Sq << a.pack_shift);  // a job shorter than one item has no rows past Sq
-    fwd_split_merge_kernel<<<dim3(split.slots / split.nsplit, (rows + 31) / 32), 256, 0, stream>>>(m);
-    if (!cuda_ok(cudaGetLastError(), "launch fwd_split_merge_kernel")) return MB_E_CUDA;
+    cudaLaunchAttribute serial;
+    serial.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    serial.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(split.slots / split.nsplit, (rows + kMergeRows - 1) / kMergeRows);
+    cfg.blockDim = dim3(256);
+    cfg.stream = stream;
+    cfg.attrs = &serial;
+    cfg.numAttrs = 1;
+    if (!cuda_ok(cudaLaunchKernelEx(&cfg, fwd_split_merge_kernel, m), "launch fwd_split_merge_kernel")) return MB_E_CUDA;
   }
   return MB_SUCCESS;
 }
