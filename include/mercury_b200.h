@@ -168,6 +168,10 @@ typedef struct mb_bwd_preprocess_args {
  * utils/attn_bwd_dsl.py:91-92). */
 MB_API int mb_attn_bwd_preprocess(const mb_bwd_preprocess_args* args, void* cuda_stream);
 
+/* mb_attn_bwd_preprocess and, in the same pass over the rows, zeroes in dq_accum [batch, hq, stat_pad, head_dim]
+ * (16-byte aligned): what MB_BWD_MODE_FUSED adds into. */
+MB_API int mb_attn_bwd_prepare_sweep(const mb_bwd_preprocess_args* args, float* dq_accum, void* cuda_stream);
+
 #define MB_BWD_MODE_DKV 1 /* owner = one K/V shard, stream = query shards: writes dK (out1) and dV (out2) */
 #define MB_BWD_MODE_DQ 0  /* owner = one query shard, stream = K/V shards: writes dQ (out1) */
 #define MB_BWD_MODE_FUSED 2 /* like DKV, and each streamed query shard's dQ contributions are ADDED (fp32,

@@ -307,6 +307,7 @@ _SIGNATURES = {
     "mb_attn_fwd_ws": [C.POINTER(AttnFwdArgs), C.c_void_p, C.c_uint64, C.c_void_p],
     "mb_attn_fwd_multi": [C.POINTER(AttnFwdMultiArgs), C.c_void_p],
     "mb_attn_bwd_preprocess": [C.POINTER(BwdPreprocessArgs), C.c_void_p],
+    "mb_attn_bwd_prepare_sweep": [C.POINTER(BwdPreprocessArgs), C.c_void_p, C.c_void_p],
     "mb_attn_bwd": [C.POINTER(AttnBwdArgs), C.c_void_p],
     "mb_attn_bwd_dq_convert": [C.c_void_p, C.c_void_p, C.c_int64, C.c_int64, C.c_int64, C.c_int32, C.c_int32, C.c_int32,
                                C.c_int32, C.c_int32, C.c_float, C.c_void_p],

@@ -209,9 +209,10 @@ def _pad64(n: int) -> int:
 
 
 def bwd_preprocess(dout: torch.Tensor, out: torch.Tensor, lse: torch.Tensor,
-                   workspace: Optional[torch.Tensor] = None) -> RowStats:
+                   workspace: Optional[torch.Tensor] = None, dq_accum: Optional[torch.Tensor] = None) -> RowStats:
     """Per-row statistics for the backward kernels.  `out` and `lse` are the FINAL forward results
-    of these query rows.  workspace: optional fp32 [2, batch, hq, pad64(sq)] to write into."""
+    of these query rows.  workspace: optional fp32 [2, batch, hq, pad64(sq)] to write into.
+    dq_accum: optional fp32 [batch, hq, pad64(sq), d] that is zeroed in the same pass (for attn_bwd_fused)."""
     _check_bshd(dout, "dout")
     _check_bshd(out, "out")
     b, sq, hq, d = dout.shape
@@ -230,8 +231,15 @@ def bwd_preprocess(dout: torch.Tensor, out: torch.Tensor, lse: torch.Tensor,
     a.out_stride_b, a.out_stride_s, a.out_stride_h = out.stride(0), out.stride(1), out.stride(2)
     a.lse, a.lse2, a.delta = lse.data_ptr(), workspace[0].data_ptr(), workspace[1].data_ptr()
     a.batch, a.sq, a.hq, a.head_dim, a.stat_pad = b, sq, hq, d, pad
+    if dq_accum is not None and (tuple(dq_accum.shape) != (b, hq, pad, d) or dq_accum.dtype != torch.float32
+                                 or not dq_accum.is_contiguous()):
+        raise ValueError(f"dq_accum must be contiguous fp32 {(b, hq, pad, d)}")
     with torch.cuda.device(dout.device):
-        _lib.check(_lib.lib.mb_attn_bwd_preprocess(C.byref(a), C.c_void_p(_stream_ptr())), "mb_attn_bwd_preprocess")
+        if dq_accum is None:
+            _lib.check(_lib.lib.mb_attn_bwd_preprocess(C.byref(a), C.c_void_p(_stream_ptr())), "mb_attn_bwd_preprocess")
+        else:
+            _lib.check(_lib.lib.mb_attn_bwd_prepare_sweep(C.byref(a), dq_accum.data_ptr(), C.c_void_p(_stream_ptr())),
+                       "mb_attn_bwd_prepare_sweep")
     return RowStats(workspace[0], workspace[1], sq)
 
 

@@ -90,7 +90,12 @@ int mb_status_peek_async(int32_t* pinned_host_dst, void* cuda_stream) {
 }
 
 int mb_attn_bwd_preprocess(const mb_bwd_preprocess_args* args, void* cuda_stream) {
-  return mb::launch_bwd_preprocess(args, static_cast<cudaStream_t>(cuda_stream));
+  return mb::launch_bwd_preprocess(args, nullptr, static_cast<cudaStream_t>(cuda_stream));
+}
+
+int mb_attn_bwd_prepare_sweep(const mb_bwd_preprocess_args* args, float* dq_accum, void* cuda_stream) {
+  if (dq_accum == nullptr || (reinterpret_cast<uintptr_t>(dq_accum) & 15u)) return MB_E_INVALID;
+  return mb::launch_bwd_preprocess(args, dq_accum, static_cast<cudaStream_t>(cuda_stream));
 }
 
 int mb_attn_bwd(const mb_attn_bwd_args* args, void* cuda_stream) {

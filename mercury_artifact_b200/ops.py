@@ -16,7 +16,7 @@ from typing import Optional, Tuple
 import torch
 
 from . import _lib
-from .attention import (_stream_ptr, attn_bwd_dkv, attn_bwd_dq, attn_bwd_fused, attn_fwd_segments,
+from .attention import (_pad64, _stream_ptr, attn_bwd_dkv, attn_bwd_dq, attn_bwd_fused, attn_fwd_segments,
                         bwd_preprocess)
 
 
@@ -121,13 +121,16 @@ def _flash_attn_backward(
     if dv is None:
         dv = torch.empty_like(v)
     q_off = k.shape[1] - q.shape[1] if causal else 0
-    stats = bwd_preprocess(dout, out, softmax_lse)
     if deterministic or q.shape[1] == 0 or k.shape[1] == 0:
+        stats = bwd_preprocess(dout, out, softmax_lse)
         attn_bwd_dq(q, dout, stats, [(k, v, 0)], softmax_scale, causal=bool(causal), q_off=q_off, dq=dq)
         attn_bwd_dkv(k, v, [(q, dout, stats, q_off)], softmax_scale, causal=bool(causal), k_off=0, dk=dk, dv=dv)
     else:
+        b, sq, hq, d = q.shape
+        acc = torch.empty((b, hq, _pad64(sq), d), dtype=torch.float32, device=q.device)
+        stats = bwd_preprocess(dout, out, softmax_lse, dq_accum=acc)
         attn_bwd_fused(q, dout, stats, k, v, softmax_scale, causal=bool(causal), q_off=q_off, k_off=0, dq=dq, dk=dk,
-                       dv=dv)
+                       dv=dv, dq_accum=acc)
     return stats.delta
 
 

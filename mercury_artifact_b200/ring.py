@@ -660,8 +660,8 @@ class RingAttention:
         L = self.seq_local
         me = self.rank
         if self.world == 1:
-            stats = bwd_preprocess(dout, o, lse)
             if self.deterministic_backward:
+                stats = bwd_preprocess(dout, o, lse)
                 attn_bwd_dq(q, dout, stats, [(kv[0], kv[1], 0)], softmax_scale, causal=self.causal, q_off=0, dq=dq)
                 attn_bwd_dkv(kv[0], kv[1], [(q, dout, stats, 0)], softmax_scale, causal=self.causal, k_off=0,
                              dk=dkv[0], dv=dkv[1])
@@ -670,7 +670,7 @@ class RingAttention:
                 if getattr(self, "_dq_accum", None) is None:
                     self._dq_accum = torch.empty((self.batch, self.hq, self.stat_pad, self.head_dim),
                                                  dtype=torch.float32, device=q.device)
-                self._dq_accum.zero_()
+                stats = bwd_preprocess(dout, o, lse, dq_accum=self._dq_accum)
                 attn_bwd_fused(q, dout, stats, kv[0], kv[1], softmax_scale, causal=self.causal, q_off=0, k_off=0,
                                dq=dq, dk=dkv[0], dv=dkv[1], dq_accum=self._dq_accum)
             self._monitor.post(torch.cuda.current_stream())

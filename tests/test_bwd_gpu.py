@@ -256,3 +256,30 @@ def test_single_sweep_with_eight_query_segments_like_one_rank_of_eight(causal):
         got = got.float().cpu()
         assert not torch.isnan(got).any()
         assert (got - want).abs().max().item() <= G_TOL
+
+
+@pytest.mark.parametrize("Sq,shift", [(1, 0), (33, 0), (64, 0), (97, 4), (200, 0)])
+def test_row_statistics_and_zeroed_dq_buffer(Sq, shift):
+    """bwd_preprocess: rows past a block of 32 and past Sq, rows that start on 8 instead of 16 bytes, and the dQ
+    buffer zeroed in the same pass.  The products are exact in fp32, a row's sum of 128 of them is off by at
+    most 128 * 2^-24 of the sum of their absolute values."""
+    from mercury_artifact_b200.attention import _pad64, bwd_preprocess
+
+    B, H, D = 2, 3, 128
+    g = torch.Generator().manual_seed(Sq)
+    do, wide = (torch.randn(B, Sq, H, D + 8, generator=g).bfloat16() for _ in range(2))
+    do, o = do[..., :D].contiguous().cuda(), wide.cuda()[..., shift:shift + D]
+    lse = torch.randn(B, H, Sq, generator=g)
+    lse[0, 0, 0] = float("-inf")
+    pad = _pad64(Sq)
+    acc = torch.full((B, H, pad, D), float("nan"), device="cuda")
+    st = bwd_preprocess(do, o, lse.cuda(), dq_accum=acc)
+    prod = (do.double() * o.double()).transpose(1, 2)
+    err = (st.delta[:, :, :Sq].double() - prod.sum(-1)).abs()
+    assert (err <= 128 * 2.0 ** -24 * prod.abs().sum(-1)).all()
+    want = torch.where(lse == float("-inf"), lse, -lse * 1.4426950408889634).cuda()
+    assert torch.equal(st.lse2[:, :, :Sq].isneginf(), want.isneginf())
+    fin = ~want.isneginf()
+    assert (st.lse2[:, :, :Sq][fin] - want[fin]).abs().max().item() <= 1e-6 * 8 if fin.any() else True
+    assert st.lse2[:, :, Sq:].isneginf().all() and (st.delta[:, :, Sq:] == 0).all()
+    assert (acc == 0).all()
