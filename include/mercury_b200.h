@@ -279,6 +279,11 @@ typedef struct mb_attn_bwd_block_args {
  * calls queued on one stream are safe.  Inputs and outputs are the caller's, as elsewhere. */
 MB_API int mb_attn_bwd_block_noalloc(const mb_attn_bwd_block_args* args, void* cuda_stream);
 
+/* Block backward in one sweep (MB_BWD_MODE_FUSED) as one call: mb_attn_bwd_prepare_sweep, mb_attn_bwd and
+ * mb_attn_bwd_dq_convert over the caller's scratch, stats [2, batch, hq, pad64(sq)] (written: lse2, then delta)
+ * and dq_accum [batch, hq, pad64(sq), head_dim] (16-byte aligned), both fp32.  sq and sk must not be 0. */
+MB_API int mb_attn_bwd_block_sweep(const mb_attn_bwd_block_args* args, float* stats, float* dq_accum, void* cuda_stream);
+
 #define MB_DTYPE_BF16 0
 #define MB_DTYPE_F32 1
 

@@ -6,6 +6,7 @@ call returns a non-zero code.
 """
 from __future__ import annotations
 
+import collections
 import ctypes as C
 from pathlib import Path
 
@@ -311,6 +312,7 @@ _SIGNATURES = {
     "mb_attn_bwd": [C.POINTER(AttnBwdArgs), C.c_void_p],
     "mb_attn_bwd_dq_convert": [C.c_void_p, C.c_void_p, C.c_int64, C.c_int64, C.c_int64, C.c_int32, C.c_int32, C.c_int32,
                                C.c_int32, C.c_int32, C.c_float, C.c_void_p],
+    "mb_attn_bwd_block_sweep": [C.POINTER(AttnBwdBlockArgs), C.c_void_p, C.c_void_p, C.c_void_p],
     "mb_attn_bwd_block_noalloc": [C.POINTER(AttnBwdBlockArgs), C.c_void_p],
     "mb_merge_out_lse": [C.POINTER(MergeArgs), C.c_void_p],
     "mb_tree_merge": [C.POINTER(C.c_void_p), C.c_int32, C.c_void_p, C.c_int64, C.c_int32, C.c_void_p],
@@ -419,29 +421,33 @@ class StatusMonitor:
         import torch
 
         self._torch = torch
-        self._slots = []   # (pinned int32 tensor, event recorded behind the copy into it)
-        self._free = []
+        # per (device, stream), oldest first: (pinned int32 tensor, event recorded behind the copy into it).  The
+        # copies of a stream complete in order, so only the oldest one has to be asked (with many calls in
+        # flight, asking all of them was most of a small call's host time).
+        self._slots = {}
+        self._free = {}   # per device: pairs to use again
         self._bad = 0
 
     def _reap(self) -> None:
-        keep = []
-        for host, ev in self._slots:
-            if ev.query():
+        for (device, _), slots in self._slots.items():
+            while slots and slots[0][1].query():
+                host, ev = slots.popleft()
                 self._bad = self._bad or int(host.item())
-                self._free.append(host)
-            else:
-                keep.append((host, ev))
-        self._slots = keep
+                self._free.setdefault(device, []).append((host, ev))
+        self._slots = {k: v for k, v in self._slots.items() if v}
 
     def post(self, stream) -> None:
         torch = self._torch
         self._reap()
-        host = self._free.pop() if self._free else torch.zeros(1, dtype=torch.int32).pin_memory()
+        free = self._free.get(stream.device_index)
+        if free:
+            host, ev = free.pop()
+        else:
+            host, ev = torch.zeros(1, dtype=torch.int32).pin_memory(), torch.cuda.Event()
         check(lib.mb_status_peek_async(C.c_void_p(host.data_ptr()), C.c_void_p(stream.cuda_stream)),
               "mb_status_peek_async")
-        ev = torch.cuda.Event()
         ev.record(stream)
-        self._slots.append((host, ev))
+        self._slots.setdefault((stream.device_index, stream.cuda_stream), collections.deque()).append((host, ev))
 
     def poll(self) -> None:
         self._reap()

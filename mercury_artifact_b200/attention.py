@@ -4,6 +4,7 @@ Tensors are torch CUDA tensors; torch is used for memory and streams only.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes as C
 from typing import Optional, Sequence, Tuple
 
@@ -12,8 +13,17 @@ import torch
 from . import _lib
 
 
+_SAME_DEVICE = contextlib.nullcontext()
+
+
+def _on(device: torch.device):
+    """torch.cuda.device(device), or nothing where that device is the current one."""
+    return _SAME_DEVICE if device.index == torch._C._cuda_getDevice() else torch.cuda.device(device)
+
+
 def _stream_ptr() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """The current stream of the current device."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _check_bshd(t: torch.Tensor, name: str) -> None:
@@ -67,12 +77,12 @@ def attn_fwd_segments(
             lse = torch.empty((b, hq, sq), dtype=torch.float32, device=q.device)
         elif lse.dtype != torch.float32 or lse.stride(2) != 1 or tuple(lse.shape) != (b, hq, sq):
             raise ValueError("lse must be an fp32 [batch, hq, sq] tensor with contiguous rows")
-        out_raw = (out.data_ptr(), out.stride(0), out.stride(1), out.stride(2))
-        lse_raw = (lse.data_ptr(), lse.stride(0), lse.stride(1))
+        out_raw = (out.data_ptr(), *out.stride()[:3])
+        lse_raw = (lse.data_ptr(), *lse.stride()[:2])
 
     args = _lib.AttnFwdArgs()
     args.q = q.data_ptr()
-    args.q_stride_b, args.q_stride_s, args.q_stride_h = q.stride(0), q.stride(1), q.stride(2)
+    args.q_stride_b, args.q_stride_s, args.q_stride_h, _ = q.stride()
     args.o, args.o_stride_b, args.o_stride_s, args.o_stride_h = out_raw
     args.lse, args.lse_stride_b, args.lse_stride_h = lse_raw
     args.batch, args.sq, args.hq, args.head_dim = b, sq, hq, d
@@ -87,29 +97,30 @@ def attn_fwd_segments(
         flag_ptr, flag_value = (segment[3], segment[4]) if len(segment) >= 5 and segment[3] else (None, 0)
         _check_bshd(k, "k")
         _check_bshd(v, "v")
-        if k.shape != v.shape or k.stride() != v.stride():
+        shape, stride = k.shape, k.stride()
+        if shape != v.shape or stride != v.stride():
             raise ValueError("k and v of one segment must share shape and strides")
-        if k.shape[0] != b or k.shape[3] != d:
+        if shape[0] != b or shape[3] != d:
             raise ValueError("segment batch/head_dim mismatch with q")
         if hkv is None:
-            hkv = k.shape[2]
-        elif hkv != k.shape[2]:
+            hkv = shape[2]
+        elif hkv != shape[2]:
             raise ValueError("all segments must have the same number of K/V heads")
         seg = args.seg[i]
         seg.k, seg.v = k.data_ptr(), v.data_ptr()
-        seg.stride_b, seg.stride_s, seg.stride_h = k.stride(0), k.stride(1), k.stride(2)
-        seg.sk = k.shape[1]
+        seg.stride_b, seg.stride_s, seg.stride_h, _ = stride
+        seg.sk = shape[1]
         seg.k_off = int(k_off)
         seg.ready_flag = flag_ptr
         seg.ready_value = int(flag_value)
     args.hkv = hkv if hkv is not None else hq
-    with torch.cuda.device(q.device):
+    with _on(q.device):
         # scratch of a launch that splits items over their keys (results in another GPU's memory are written by
         # the attention kernel itself); freed in stream order by the caching allocator
         need = 0 if raw else _lib.lib.mb_attn_fwd_workspace(C.byref(args))
         ws = torch.empty(need, dtype=torch.uint8, device=q.device) if need > 0 else None
         _lib.check(_lib.lib.mb_attn_fwd_ws(C.byref(args), ws.data_ptr() if need > 0 else None, need,
-                                           C.c_void_p(_stream_ptr())), "mb_attn_fwd_ws")
+                                           _stream_ptr()), "mb_attn_fwd_ws")
     return (None, None) if raw else (out, lse)
 
 
@@ -188,8 +199,8 @@ def attn_fwd_multi(jobs: Sequence[dict], segments: Sequence[tuple], softmax_scal
         seg.stride_b, seg.stride_s, seg.stride_h = k.stride(0), k.stride(1), k.stride(2)
         seg.sk, seg.k_off = k.shape[1], int(k_off)
         seg.ready_flag, seg.ready_value = flag_ptr, int(flag_value)
-    with torch.cuda.device(device):
-        _lib.check(_lib.lib.mb_attn_fwd_multi(C.byref(a), C.c_void_p(_stream_ptr())), "mb_attn_fwd_multi")
+    with _on(device):
+        _lib.check(_lib.lib.mb_attn_fwd_multi(C.byref(a), _stream_ptr()), "mb_attn_fwd_multi")
 
 
 # ------------------------------------------------------------------------------------------
@@ -234,11 +245,11 @@ def bwd_preprocess(dout: torch.Tensor, out: torch.Tensor, lse: torch.Tensor,
     if dq_accum is not None and (tuple(dq_accum.shape) != (b, hq, pad, d) or dq_accum.dtype != torch.float32
                                  or not dq_accum.is_contiguous()):
         raise ValueError(f"dq_accum must be contiguous fp32 {(b, hq, pad, d)}")
-    with torch.cuda.device(dout.device):
+    with _on(dout.device):
         if dq_accum is None:
-            _lib.check(_lib.lib.mb_attn_bwd_preprocess(C.byref(a), C.c_void_p(_stream_ptr())), "mb_attn_bwd_preprocess")
+            _lib.check(_lib.lib.mb_attn_bwd_preprocess(C.byref(a), _stream_ptr()), "mb_attn_bwd_preprocess")
         else:
-            _lib.check(_lib.lib.mb_attn_bwd_prepare_sweep(C.byref(a), dq_accum.data_ptr(), C.c_void_p(_stream_ptr())),
+            _lib.check(_lib.lib.mb_attn_bwd_prepare_sweep(C.byref(a), dq_accum.data_ptr(), _stream_ptr()),
                        "mb_attn_bwd_prepare_sweep")
     return RowStats(workspace[0], workspace[1], sq)
 
@@ -300,8 +311,8 @@ def _bwd_launch(mode, own, own_g, own_off, segments, hq, hkv, scale, causal, out
             if acc.dtype != torch.float32 or not acc.is_contiguous() or tuple(acc.shape) != (b, hq, seg.stat_pad, d):
                 raise ValueError(f"dq_accum must be contiguous fp32 {(b, hq, seg.stat_pad, d)}")
             seg.dq_accum = acc.data_ptr()
-    with torch.cuda.device(own.device):
-        _lib.check(_lib.lib.mb_attn_bwd(C.byref(a), C.c_void_p(_stream_ptr())), "mb_attn_bwd")
+    with _on(own.device):
+        _lib.check(_lib.lib.mb_attn_bwd(C.byref(a), _stream_ptr()), "mb_attn_bwd")
 
 
 def attn_bwd_dq(q, dout, stats: RowStats, kv_segments, softmax_scale, causal=False, q_off=0, dq=None,
@@ -345,10 +356,10 @@ def dq_convert_raw(dq_accum: torch.Tensor, dq_ptr: int, strides: Sequence[int], 
     """Finish a single-sweep backward: scale the fp32 dq accumulation [batch, hq, pad, d] and store it as
     [batch, sq, hq, d] rows at a raw address with element strides (batch, row, head) -- the address may
     be another rank's memory mapped into this process (mb_attn_bwd_dq_convert)."""
-    with torch.cuda.device(dq_accum.device):
+    with _on(dq_accum.device):
         _lib.check(_lib.lib.mb_attn_bwd_dq_convert(dq_accum.data_ptr(), dq_ptr, strides[0], strides[1], strides[2],
                                                    batch, sq, hq, pad, _OUT_MODES[out_dtype], float(softmax_scale),
-                                                   C.c_void_p(_stream_ptr())),
+                                                   _stream_ptr()),
                    "mb_attn_bwd_dq_convert")
 
 
@@ -372,9 +383,59 @@ def attn_bwd_fused(q, dout, stats: RowStats, k, v, softmax_scale, causal=False, 
     _bwd_launch(_lib.MB_BWD_MODE_FUSED, k, v, k_off, [seg], hq, k.shape[2], softmax_scale, causal, dk, dv, False)
     if dq.dtype not in _OUT_MODES or dq.stride(3) != 1 or tuple(dq.shape) != tuple(q.shape):
         raise ValueError("dq must be bf16 or fp32, shaped like q, with a contiguous head_dim")
-    with torch.cuda.device(q.device):
+    with _on(q.device):
         _lib.check(_lib.lib.mb_attn_bwd_dq_convert(dq_accum.data_ptr(), dq.data_ptr(), dq.stride(0), dq.stride(1),
                                                    dq.stride(2), b, sq, hq, stats.pad, _OUT_MODES[dq.dtype],
-                                                   float(softmax_scale), C.c_void_p(_stream_ptr())),
+                                                   float(softmax_scale), _stream_ptr()),
                    "mb_attn_bwd_dq_convert")
     return dq, dk, dv
+
+
+def _one_call_sweep(dout, q, k, v, out, lse, dq, dk, dv) -> bool:
+    """Whether attn_bwd_block can hand these tensors to mb_attn_bwd_block_sweep as they are."""
+    shape, stride, kv_shape, g_stride = q.shape, q.stride(), k.shape, dk.stride()
+    bf16 = torch.bfloat16
+    return (len(shape) == 4 and len(kv_shape) == 4 and dout.shape == shape and out.shape == shape and v.shape == kv_shape
+            and kv_shape[0] == shape[0] and kv_shape[3] == shape[3] and min(shape) > 0 and min(kv_shape) > 0
+            and shape[2] % kv_shape[2] == 0
+            and dout.stride() == stride and out.stride() == stride and stride[3] == 1
+            and k.stride() == v.stride() and k.stride(3) == 1
+            and q.dtype == dout.dtype == out.dtype == k.dtype == v.dtype == bf16
+            and lse.dtype == torch.float32 and lse.is_contiguous() and lse.shape == (shape[0], shape[2], shape[1])
+            and dq.shape == shape and dq.stride(3) == 1
+            and dk.shape == kv_shape and dv.shape == kv_shape and dv.stride() == g_stride and g_stride[3] == 1
+            and dq.dtype == dk.dtype == dv.dtype and dq.dtype in _OUT_MODES
+            and q.is_cuda and q.device == dout.device == out.device == k.device == v.device == lse.device == dq.device
+            == dk.device == dv.device)
+
+
+def attn_bwd_block(dout, q, k, v, out, lse, softmax_scale, causal, q_off, k_off, dq, dk, dv,
+                   dq_accum: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """bwd_preprocess and attn_bwd_fused of one (query shard, K/V shard) pair; returns delta [batch, hq, pad64(sq)].
+    One library call where the tensors share strides as the block entry takes them, else the two functions."""
+    b, sq, hq, d = q.shape
+    pad = _pad64(sq)
+    if dq_accum is None:
+        dq_accum = torch.empty((b, hq, pad, d), dtype=torch.float32, device=q.device)
+    if not _one_call_sweep(dout, q, k, v, out, lse, dq, dk, dv):
+        stats = bwd_preprocess(dout, out, lse, dq_accum=dq_accum)
+        attn_bwd_fused(q, dout, stats, k, v, softmax_scale, causal=causal, q_off=q_off, k_off=k_off, dq=dq, dk=dk, dv=dv,
+                       dq_accum=dq_accum)
+        return stats.delta
+    if tuple(dq_accum.shape) != (b, hq, pad, d) or dq_accum.dtype != torch.float32 or not dq_accum.is_contiguous():
+        raise ValueError(f"dq_accum must be contiguous fp32 {(b, hq, pad, d)}")
+    stats = torch.empty((2, b, hq, pad), dtype=torch.float32, device=q.device)
+    a = _lib.AttnBwdBlockArgs()
+    a.dout, a.q, a.out, a.k, a.v = dout.data_ptr(), q.data_ptr(), out.data_ptr(), k.data_ptr(), v.data_ptr()
+    a.q_stride_b, a.q_stride_s, a.q_stride_h, _ = q.stride()
+    a.kv_stride_b, a.kv_stride_s, a.kv_stride_h, _ = k.stride()
+    a.lse, a.dq, a.dk, a.dv = lse.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr()
+    a.dq_stride_b, a.dq_stride_s, a.dq_stride_h, _ = dq.stride()
+    a.dkv_stride_b, a.dkv_stride_s, a.dkv_stride_h, _ = dk.stride()
+    a.batch, a.sq, a.sk, a.hq, a.hkv, a.head_dim = b, sq, k.shape[1], hq, k.shape[2], d
+    a.q_off, a.k_off, a.causal = int(q_off), int(k_off), 1 if causal else 0
+    a.out_mode, a.softmax_scale = _OUT_MODES[dq.dtype], float(softmax_scale)
+    with _on(q.device):
+        _lib.check(_lib.lib.mb_attn_bwd_block_sweep(C.byref(a), stats.data_ptr(), dq_accum.data_ptr(), _stream_ptr()),
+                   "mb_attn_bwd_block_sweep")
+    return stats[1]

@@ -554,6 +554,75 @@ int launch_attn_bwd(const mb_attn_bwd_args* x, cudaStream_t stream) {
 }
 
 // ---------------------------------------------------------------------------
+// block backward, one sweep, in one call
+// ---------------------------------------------------------------------------
+static bool block_args_ok(const mb_attn_bwd_block_args* x, int* rc) {
+  *rc = MB_E_INVALID;
+  if (x == nullptr) return false;
+  if (x->head_dim != kBD) {
+    *rc = MB_E_UNSUPPORTED;
+    return false;
+  }
+  if (x->batch <= 0 || x->hq <= 0 || x->hkv <= 0 || x->hq % x->hkv != 0 || x->sq < 0 || x->sk < 0) return false;
+  if (x->out_mode != MB_OUT_BF16 && x->out_mode != MB_OUT_F32) return false;
+  return x->dout != nullptr && x->q != nullptr && x->k != nullptr && x->v != nullptr && x->out != nullptr &&
+         x->lse != nullptr && x->dq != nullptr && x->dk != nullptr && x->dv != nullptr;
+}
+
+// Statistics (dout and out with q's strides) and, with dq_accum, the zeroed dQ buffer.
+static int block_preprocess(const mb_attn_bwd_block_args* x, float* lse2, float* delta, int stat_pad, float* dq_accum,
+                            cudaStream_t stream) {
+  mb_bwd_preprocess_args p;
+  memset(&p, 0, sizeof(p));
+  p.dout = x->dout; p.dout_stride_b = x->q_stride_b; p.dout_stride_s = x->q_stride_s; p.dout_stride_h = x->q_stride_h;
+  p.out = x->out; p.out_stride_b = x->q_stride_b; p.out_stride_s = x->q_stride_s; p.out_stride_h = x->q_stride_h;
+  p.lse = x->lse; p.lse2 = lse2; p.delta = delta;
+  p.batch = x->batch; p.sq = x->sq; p.hq = x->hq; p.head_dim = x->head_dim; p.stat_pad = stat_pad;
+  return launch_bwd_preprocess(&p, dq_accum, stream);
+}
+
+// Owner K/V, stream q/dout: modes DKV and FUSED.
+static void block_owner_kv(const mb_attn_bwd_block_args* x, float* lse2, float* delta, int stat_pad, float* dq_accum,
+                           mb_attn_bwd_args* a) {
+  a->own = x->k; a->own_g = x->v;
+  a->own_stride_b = x->kv_stride_b; a->own_stride_s = x->kv_stride_s; a->own_stride_h = x->kv_stride_h;
+  a->own_lse2 = nullptr; a->own_delta = nullptr; a->own_stat_pad = 0;
+  a->own_rows = x->sk; a->own_off = x->k_off;
+  a->out1 = x->dk; a->out2 = x->dv;
+  a->out_stride_b = x->dkv_stride_b; a->out_stride_s = x->dkv_stride_s; a->out_stride_h = x->dkv_stride_h;
+  a->nseg = 1;
+  a->seg[0].str = x->q; a->seg[0].str_g = x->dout;
+  a->seg[0].stride_b = x->q_stride_b; a->seg[0].stride_s = x->q_stride_s; a->seg[0].stride_h = x->q_stride_h;
+  a->seg[0].rows = x->sq; a->seg[0].pos_off = x->q_off;
+  a->seg[0].lse2 = lse2; a->seg[0].delta = delta; a->seg[0].stat_pad = stat_pad;
+  a->seg[0].dq_accum = dq_accum;
+}
+
+int launch_bwd_block_sweep(const mb_attn_bwd_block_args* x, float* stats, float* dq_accum, cudaStream_t stream) {
+  int rc;
+  if (!block_args_ok(x, &rc)) return rc;
+  if (x->sq == 0 || x->sk == 0 || stats == nullptr || dq_accum == nullptr ||
+      (reinterpret_cast<uintptr_t>(dq_accum) & 15u))
+    return MB_E_INVALID;
+  const long long pad = (x->sq + (long long)kStrRows - 1) / kStrRows * kStrRows;
+  if (pad > INT_MAX) return MB_E_INVALID;
+  float* lse2 = stats;
+  float* delta = stats + (long long)x->batch * x->hq * pad;
+  rc = block_preprocess(x, lse2, delta, (int)pad, dq_accum, stream);
+  if (rc != MB_SUCCESS) return rc;
+  static thread_local mb_attn_bwd_args a;
+  memset(&a, 0, sizeof(a));
+  a.batch = x->batch; a.hq = x->hq; a.hkv = x->hkv; a.head_dim = x->head_dim;
+  a.causal = x->causal; a.softmax_scale = x->softmax_scale; a.out_mode = x->out_mode; a.status = x->status;
+  a.mode = MB_BWD_MODE_FUSED;
+  block_owner_kv(x, lse2, delta, (int)pad, dq_accum, &a);
+  rc = launch_attn_bwd(&a, stream);
+  if (rc != MB_SUCCESS) return rc;
+  return launch_dq_convert(dq_accum, x->dq, x->dq_stride_b, x->dq_stride_s, x->dq_stride_h, x->batch, x->sq, x->hq,
+                           (int)pad, x->out_mode, x->softmax_scale, stream);
+}
+
+// ---------------------------------------------------------------------------
 // allocation-free block backward
 // ---------------------------------------------------------------------------
 // Row statistics (lse2, delta) for the allocation-free entry point live in this fixed array
@@ -584,18 +653,12 @@ static float* static_stats_address(int* rc) {
 }
 
 int launch_bwd_block_noalloc(const mb_attn_bwd_block_args* x, cudaStream_t stream) {
-  if (x == nullptr) return MB_E_INVALID;
-  if (x->head_dim != kBD) return MB_E_UNSUPPORTED;
-  if (x->batch <= 0 || x->hq <= 0 || x->hkv <= 0 || x->hq % x->hkv != 0 || x->sq < 0 || x->sk < 0) return MB_E_INVALID;
-  if (x->out_mode != MB_OUT_BF16 && x->out_mode != MB_OUT_F32) return MB_E_INVALID;
-  if (x->dout == nullptr || x->q == nullptr || x->k == nullptr || x->v == nullptr || x->out == nullptr ||
-      x->lse == nullptr || x->dq == nullptr || x->dk == nullptr || x->dv == nullptr)
-    return MB_E_INVALID;
+  int rc = MB_SUCCESS;
+  if (!block_args_ok(x, &rc)) return rc;
   const long long pad = (x->sq + kStrRows - 1) / kStrRows * (long long)kStrRows;
   const long long rows = (long long)x->batch * x->hq * (pad > 0 ? pad : kStrRows);
   if (rows > kStaticStatRows) return MB_E_TOO_LARGE;
   if (x->sq == 0 && x->sk == 0) return MB_SUCCESS;
-  int rc = MB_SUCCESS;
   float* stats = static_stats_address(&rc);
   if (stats == nullptr) return rc;
   const int stat_pad = static_cast<int>(pad > 0 ? pad : kStrRows);
@@ -603,13 +666,7 @@ int launch_bwd_block_noalloc(const mb_attn_bwd_block_args* x, cudaStream_t strea
   float* delta = stats + kStaticStatRows;
 
   if (x->sq > 0) {
-    mb_bwd_preprocess_args p;
-    memset(&p, 0, sizeof(p));
-    p.dout = x->dout; p.dout_stride_b = x->q_stride_b; p.dout_stride_s = x->q_stride_s; p.dout_stride_h = x->q_stride_h;
-    p.out = x->out; p.out_stride_b = x->q_stride_b; p.out_stride_s = x->q_stride_s; p.out_stride_h = x->q_stride_h;
-    p.lse = x->lse; p.lse2 = lse2; p.delta = delta;
-    p.batch = x->batch; p.sq = x->sq; p.hq = x->hq; p.head_dim = x->head_dim; p.stat_pad = stat_pad;
-    rc = launch_bwd_preprocess(&p, nullptr, stream);
+    rc = block_preprocess(x, lse2, delta, stat_pad, nullptr, stream);
     if (rc != MB_SUCCESS) return rc;
   }
 
@@ -633,16 +690,7 @@ int launch_bwd_block_noalloc(const mb_attn_bwd_block_args* x, cudaStream_t strea
   if (rc != MB_SUCCESS) return rc;
   // dK/dV: owner = k/v, stream = q/dout with the statistics just computed
   a.mode = MB_BWD_MODE_DKV;
-  a.own = x->k; a.own_g = x->v;
-  a.own_stride_b = x->kv_stride_b; a.own_stride_s = x->kv_stride_s; a.own_stride_h = x->kv_stride_h;
-  a.own_lse2 = nullptr; a.own_delta = nullptr; a.own_stat_pad = 0;
-  a.own_rows = x->sk; a.own_off = x->k_off;
-  a.out1 = x->dk; a.out2 = x->dv;
-  a.out_stride_b = x->dkv_stride_b; a.out_stride_s = x->dkv_stride_s; a.out_stride_h = x->dkv_stride_h;
-  a.seg[0].str = x->q; a.seg[0].str_g = x->dout;
-  a.seg[0].stride_b = x->q_stride_b; a.seg[0].stride_s = x->q_stride_s; a.seg[0].stride_h = x->q_stride_h;
-  a.seg[0].rows = x->sq; a.seg[0].pos_off = x->q_off;
-  a.seg[0].lse2 = lse2; a.seg[0].delta = delta; a.seg[0].stat_pad = stat_pad;
+  block_owner_kv(x, lse2, delta, stat_pad, nullptr, &a);
   return launch_attn_bwd(&a, stream);
 }
 

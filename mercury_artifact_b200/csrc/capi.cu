@@ -109,6 +109,10 @@ int mb_attn_bwd_dq_convert(const float* dq_accum, void* dq, int64_t dq_stride_b,
                                softmax_scale, static_cast<cudaStream_t>(cuda_stream));
 }
 
+int mb_attn_bwd_block_sweep(const mb_attn_bwd_block_args* args, float* stats, float* dq_accum, void* cuda_stream) {
+  return mb::launch_bwd_block_sweep(args, stats, dq_accum, static_cast<cudaStream_t>(cuda_stream));
+}
+
 int mb_attn_bwd_block_noalloc(const mb_attn_bwd_block_args* args, void* cuda_stream) {
   return mb::launch_bwd_block_noalloc(args, static_cast<cudaStream_t>(cuda_stream));
 }

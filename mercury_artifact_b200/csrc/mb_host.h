@@ -33,6 +33,7 @@ int launch_bwd_preprocess(const mb_bwd_preprocess_args* args, float* dq_accum, c
 int launch_attn_bwd(const mb_attn_bwd_args* args, cudaStream_t stream);
 int launch_dq_convert(const float* acc, void* dq, long long sb, long long ss, long long sh, int batch, int sq, int hq,
                       int pad, int out_mode, float scale, cudaStream_t stream);
+int launch_bwd_block_sweep(const mb_attn_bwd_block_args* args, float* stats, float* dq_accum, cudaStream_t stream);
 int launch_bwd_block_noalloc(const mb_attn_bwd_block_args* args, cudaStream_t stream);
 
 }  // namespace mb

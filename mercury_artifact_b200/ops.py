@@ -16,7 +16,7 @@ from typing import Optional, Tuple
 import torch
 
 from . import _lib
-from .attention import (_pad64, _stream_ptr, attn_bwd_dkv, attn_bwd_dq, attn_bwd_fused, attn_fwd_segments,
+from .attention import (_on, _stream_ptr, attn_bwd_block, attn_bwd_dkv, attn_bwd_dq, attn_fwd_segments,
                         bwd_preprocess)
 
 
@@ -126,11 +126,7 @@ def _flash_attn_backward(
         attn_bwd_dq(q, dout, stats, [(k, v, 0)], softmax_scale, causal=bool(causal), q_off=q_off, dq=dq)
         attn_bwd_dkv(k, v, [(q, dout, stats, q_off)], softmax_scale, causal=bool(causal), k_off=0, dk=dk, dv=dv)
     else:
-        b, sq, hq, d = q.shape
-        acc = torch.empty((b, hq, _pad64(sq), d), dtype=torch.float32, device=q.device)
-        stats = bwd_preprocess(dout, out, softmax_lse, dq_accum=acc)
-        attn_bwd_fused(q, dout, stats, k, v, softmax_scale, causal=bool(causal), q_off=q_off, k_off=0, dq=dq, dk=dk,
-                       dv=dv, dq_accum=acc)
+        return attn_bwd_block(dout, q, k, v, out, softmax_lse, softmax_scale, bool(causal), q_off, 0, dq, dk, dv)
     return stats.delta
 
 
@@ -154,8 +150,8 @@ def _merge_launch(out, lse, block_out, block_lse, first: bool) -> None:
     a.batch, a.seq, a.heads, a.head_dim = b, s, h, d
     a.first = 1 if first else 0
     a.block_dtype = _lib.MB_DTYPE_F32 if block_out.dtype == torch.float32 else _lib.MB_DTYPE_BF16
-    with torch.cuda.device(out.device):
-        _lib.check(_lib.lib.mb_merge_out_lse(C.byref(a), C.c_void_p(_stream_ptr())), "mb_merge_out_lse")
+    with _on(out.device):
+        _lib.check(_lib.lib.mb_merge_out_lse(C.byref(a), _stream_ptr()), "mb_merge_out_lse")
 
 
 def update_out_and_lse(
@@ -204,7 +200,7 @@ def flash_reduce(lhs: torch.Tensor, rhs: torch.Tensor) -> torch.Tensor:
     out = torch.empty_like(lhs)
     width = lhs.shape[-1]
     rows = lhs.numel() // width if width else 0
-    with torch.cuda.device(lhs.device):
+    with _on(lhs.device):
         _lib.check(_lib.lib.mb_flash_reduce(lhs.data_ptr(), rhs.data_ptr(), out.data_ptr(), rows, width,
-                                            C.c_void_p(_stream_ptr())), "mb_flash_reduce")
+                                            _stream_ptr()), "mb_flash_reduce")
     return out

@@ -39,7 +39,7 @@ from typing import Dict, List, Optional, Sequence, Tuple
 import torch
 
 from . import _lib, mesh
-from .attention import (RowStats, _bwd_launch, _pad64, attn_bwd_dkv, attn_bwd_dq, attn_bwd_fused, attn_fwd_multi,
+from .attention import (RowStats, _bwd_launch, _pad64, attn_bwd_block, attn_bwd_dkv, attn_bwd_dq, attn_fwd_multi,
                         attn_fwd_segments, bwd_preprocess, dq_convert_raw)
 from .comm import PeerContext, SymmetricBuffer, _align, default_context
 
@@ -670,9 +670,8 @@ class RingAttention:
                 if getattr(self, "_dq_accum", None) is None:
                     self._dq_accum = torch.empty((self.batch, self.hq, self.stat_pad, self.head_dim),
                                                  dtype=torch.float32, device=q.device)
-                stats = bwd_preprocess(dout, o, lse, dq_accum=self._dq_accum)
-                attn_bwd_fused(q, dout, stats, kv[0], kv[1], softmax_scale, causal=self.causal, q_off=0, k_off=0,
-                               dq=dq, dk=dkv[0], dv=dkv[1], dq_accum=self._dq_accum)
+                attn_bwd_block(dout, q, kv[0], kv[1], o, lse, softmax_scale, self.causal, 0, 0, dq, dkv[0], dkv[1],
+                               dq_accum=self._dq_accum)
             self._monitor.post(torch.cuda.current_stream())
             return dq, dkv
         if not self.with_backward:
