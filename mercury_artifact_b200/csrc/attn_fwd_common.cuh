@@ -63,6 +63,7 @@ struct FwdArgs {
   int seg_koff[MB_MAX_SEGMENTS];
   const int* seg_flag[MB_MAX_SEGMENTS];  // arrival flag of a staged shard (nullptr: already in place)
   int seg_flag_value[MB_MAX_SEGMENTS];
+  int overlap;  // launched with launch_overlapped
   int causal;
   float scale;       // softmax scale
   float scale_log2;  // softmax scale * log2(e)

@@ -39,6 +39,15 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
 }
 
 // ---------------------------------------------------------------------------
+// launches that overlap (see launch_overlapped in mb_host.h)
+// ---------------------------------------------------------------------------
+// Lets the next kernel's blocks be set up as soon as every block of this one has started; they wait for the end of
+// this kernel in grid_dependency_wait, which a kernel calls before it touches global memory.  (Every kernel that
+// may start early waits, so the end of one implies the end of all before it.)
+__device__ __forceinline__ void grid_dependents_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// ---------------------------------------------------------------------------
 // mbarrier
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {

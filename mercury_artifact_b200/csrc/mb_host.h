@@ -16,6 +16,24 @@ int encode_tiled_bf16(CUtensorMap* map, void* base, int rank, const cuuint64_t* 
 // Remember a failed CUDA runtime call for mb_last_cuda_error(); returns true when `e` is cudaSuccess.
 bool cuda_ok(cudaError_t e, const char* what);
 
+// Launches a kernel whose blocks may be set up while the previous kernel of the stream ends (programmatic
+// serialization).  The kernel calls grid_dependency_wait() before its first access to global memory.
+template <class... Params, class... Args>
+bool launch_overlapped(const char* what, void (*kernel)(Params...), dim3 grid, int threads, size_t smem,
+                       cudaStream_t stream, const Args&... args) {
+  cudaLaunchAttribute serial;
+  serial.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  serial.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &serial;
+  cfg.numAttrs = 1;
+  return cuda_ok(cudaLaunchKernelEx(&cfg, kernel, args...), what);
+}
+
 // Device address of the library's status word on the current device (nullptr on failure).
 int* default_status_word();
 

@@ -9,6 +9,7 @@
 // written per output element.
 #include <cuda_bf16.h>
 
+#include "mb_common.cuh"
 #include "mb_host.h"
 
 namespace mb {
@@ -103,6 +104,8 @@ __global__ void __launch_bounds__(256, MB_MERGE_BLOCKS_PER_SM) merge_kernel(cons
   const long long step = nwarps * kRowsPerWarp;
   float my_w;
   long long my_brow;
+  grid_dependents_launch();
+  grid_dependency_wait();
   merge_weights(a, warp0 * kRowsPerWarp, rows, lane, my_w, my_brow);
   for (long long row0 = warp0 * kRowsPerWarp; row0 < rows; row0 += step) {
     float w[kRowsPerWarp];
@@ -289,9 +292,10 @@ int launch_merge(const mb_merge_args* x, cudaStream_t stream) {
   const long long want = (rows + 8 * kRowsPerWarp - 1) / (8 * kRowsPerWarp);  // 8 warps per block
   const long long cap = static_cast<long long>(sms) * MB_MERGE_BLOCKS_PER_SM;  // one resident wave, grid-stride loop
   const int grid = static_cast<int>(want < cap ? want : cap);
-  if (a.block_is_f32) merge_kernel<true><<<grid, 256, 0, stream>>>(a);
-  else merge_kernel<false><<<grid, 256, 0, stream>>>(a);
-  return cudaGetLastError() == cudaSuccess ? MB_SUCCESS : MB_E_CUDA;
+  return launch_overlapped("launch merge_kernel", a.block_is_f32 ? merge_kernel<true> : merge_kernel<false>, dim3(grid), 256, 0,
+                           stream, a)
+             ? MB_SUCCESS
+             : MB_E_CUDA;
 }
 
 }  // namespace mb
