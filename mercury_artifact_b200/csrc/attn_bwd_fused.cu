@@ -10,10 +10,11 @@
 // plus, per step,
 //     dQ^T(step) = K^T dS^T  (rows: head-dim, columns: the 64 queries of the step)
 // which is not accumulated on chip (every step has other queries) but added into an fp32 buffer
-// [batch, hq, rows, head_dim] in global memory: the drain warps transpose it through shared memory
-// into 32 query rows x 128 floats (16 KiB, contiguous in the buffer) and one thread adds it with a
-// bulk reduction (cp.reduce.async.bulk ... add.f32).  Per-element red.global.add from registers was
-// measured first: it cost 18 % of the kernel.  Each query row receives one contribution per K/V
+// [batch, hq, rows, head_dim] in global memory: the drain warps add 24 of the 64 query rows of a step with
+// red.global.add.f32 from registers (a lane holds one head-dim index, so a warp adds 128 contiguous bytes) and
+// transpose the other 40 through shared memory into rows of 128 floats (20 KiB, contiguous in the buffer)
+// that one thread adds with a bulk reduction (cp.reduce.async.bulk ... add.f32).  Without the additions the kernel
+// would take 751 us instead of 828 (4 096 x 4 096, 32 heads).  Each query row receives one contribution per K/V
 // tile that it can see.  A small kernel afterwards scales and converts the
 // buffer to bf16.  The order of those fp32 additions varies from run to run, so dQ is not
 // bitwise reproducible (dK and dV are); the two-launch form stays available for callers that
@@ -65,7 +66,12 @@ __device__ __forceinline__ void fused_regs_ew() {
 }
 constexpr int kFusedStages = 3;
 constexpr int kDsBytes = kOwnRows * kStrRows * 2;  // 16 KiB: dS^T as [128 keys][64 queries] bf16
-constexpr int kDqStageBytes = 32 * kBD * 4;          // 16 KiB: 32 query rows x 128 floats on their way to the reduction
+// Query rows of a step that go through the staging tile and the bulk reduction; the others are added from registers.
+// The first way is limited by shared memory (a write and a read of every float), the second by the load/store path;
+// each alone takes 870 us for a block of 4 096 x 4 096 with 32 heads, shared between them: 16 rows staged 843,
+// 24 842, 32 837, 36 826, 40 828, 44 828, 48 843.
+constexpr int kDqStaged = 40;
+constexpr int kDqStageBytes = kDqStaged * kBD * 4;
 constexpr int kFusedSmemBytes =
     2 * kOwnTileBytes + kFusedStages * kBwdStageBytes + 2 * kDsBytes + kDqStageBytes + 1024 + 1024;
 static_assert(kFusedSmemBytes <= 232448, "shared memory budget of one CTA");
@@ -122,6 +128,10 @@ __device__ __forceinline__ void issue_dq_group(uint32_t d_tmem, uint64_t k_desc,
       :
       : "r"(d_tmem), "l"(k_desc), "l"(ds_desc), "r"(idesc)
       : "memory");
+}
+
+__device__ __forceinline__ void red_add(float* p, uint32_t x) {
+  asm volatile("red.global.add.f32 [%0], %1;" ::"l"(p), "f"(__uint_as_float(x)) : "memory");
 }
 
 template <int kLaunchRegs>
@@ -372,26 +382,37 @@ __global__ void __maxnreg__(kLaunchRegs) attn_bwd_fused_kernel(const __grid_cons
           tc_fence_before();
           mbar_arrive(&ctl->dq_free[t & 1]);
           const int r0 = st * kStrRows;
+          // The step's rows past the first kDqStaged are added from registers: a warp adds 128 contiguous bytes of a
+          // row.  They go first, while the previous bulk reduction reads the staging tile.
+          {
+            const int nrow = rows - (r0 + kDqStaged);  // rows past the shard's end carry zeros: skipped
+            float* dst = acc_base + (long long)(r0 + kDqStaged) * kBD + d;
+            if (nrow >= kStrRows - kDqStaged) {
 #pragma unroll
-          for (int hh = 0; hh < 2; ++hh) {
-            const int nrow = min(32, rows - (r0 + hh * 32));  // rows past the shard's end carry zeros: skipped
-            // the staging tile is free once the previous bulk reduction has read it
-            if (issuer) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-            asm volatile("bar.sync 1, 128;" ::: "memory");
-            // transpose: lane d of the tile's column e becomes element [e][d] (conflict-free rows of 128 floats)
+              for (int e = 0; e < kStrRows - kDqStaged; ++e) red_add(dst + e * kBD, v[(kDqStaged + e) >> 5][(kDqStaged + e) & 31]);
+            } else {
 #pragma unroll
-            for (int e = 0; e < 32; ++e) sDq[e * kBD + d] = __uint_as_float(v[hh][e]);
-            fence_proxy_async_smem();
-            asm volatile("bar.sync 1, 128;" ::: "memory");
-            if (issuer && nrow > 0) {
-              float* dst = acc_base + (long long)(r0 + hh * 32) * kBD;
-              asm volatile(
-                  "cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;\n\t"
-                  "cp.async.bulk.commit_group;"
-                  :
-                  : "l"(dst), "r"(smem_u32(sDq)), "r"(nrow * kBD * 4)
-                  : "memory");
+              for (int e = 0; e < kStrRows - kDqStaged; ++e)
+                if (e < nrow) red_add(dst + e * kBD, v[(kDqStaged + e) >> 5][(kDqStaged + e) & 31]);
             }
+          }
+          // the staging tile is free once the previous bulk reduction has read it
+          if (issuer) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+          asm volatile("bar.sync 1, 128;" ::: "memory");
+          // transpose: lane d of the tile's column e becomes element [e][d] (conflict-free rows of 128 floats)
+#pragma unroll
+          for (int e = 0; e < kDqStaged; ++e) sDq[e * kBD + d] = __uint_as_float(v[e >> 5][e & 31]);
+          fence_proxy_async_smem();
+          asm volatile("bar.sync 1, 128;" ::: "memory");
+          if (issuer) {
+            const int nrow = min(kDqStaged, rows - r0);
+            float* dst = acc_base + (long long)r0 * kBD;
+            asm volatile(
+                "cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;\n\t"
+                "cp.async.bulk.commit_group;"
+                :
+                : "l"(dst), "r"(smem_u32(sDq)), "r"(nrow * kBD * 4)
+                : "memory");
           }
         }
       }

@@ -283,3 +283,25 @@ def test_row_statistics_and_zeroed_dq_buffer(Sq, shift):
     assert (st.lse2[:, :, :Sq][fin] - want[fin]).abs().max().item() <= 1e-6 * 8 if fin.any() else True
     assert st.lse2[:, :, Sq:].isneginf().all() and (st.delta[:, :, Sq:] == 0).all()
     assert (acc == 0).all()
+
+
+@pytest.mark.parametrize("Sq", [1, 39, 40, 41, 63, 64, 65, 104, 105, 127])
+def test_single_sweep_rows_of_the_last_step(Sq):
+    """A step's 64 query rows reach the dQ buffer on two ways (40 through the staging tile, the others from registers):
+    every number of rows in the last step around both limits, and nothing past the last row."""
+    import mercury_artifact_b200 as mb
+    from oracle import block
+
+    B, Sk, H, D = 1, 200, 2, 128
+    q, _, _, do = seeded_qkv(31, B, Sq, H, H, D)
+    _, k, v, _ = seeded_qkv(32, B, Sk, H, H, D)
+    scale = D ** -0.5
+    ro, rl = block.block_attn_fwd(q, k, v, scale)
+    gq, gk, gv = block.block_attn_bwd(do, q, k, v, ro, rl, scale)
+    st = mb.bwd_preprocess(do.cuda(), ro.cuda(), rl.cuda())
+    acc = torch.zeros(B, H, st.pad, D, device="cuda")
+    dq, dk, dv = mb.attn_bwd_fused(q.cuda(), do.cuda(), st, k.cuda(), v.cuda(), scale, dq_accum=acc)
+    _status_ok()
+    for got, want in ((dq, gq), (dk, gk), (dv, gv)):
+        assert (got.float().cpu() - want).abs().max().item() <= G_TOL
+    assert (acc[:, :, Sq:] == 0).all()
