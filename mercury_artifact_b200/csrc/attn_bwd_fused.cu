@@ -67,9 +67,9 @@ __device__ __forceinline__ void fused_regs_ew() {
 constexpr int kFusedStages = 3;
 constexpr int kDsBytes = kOwnRows * kStrRows * 2;  // 16 KiB: dS^T as [128 keys][64 queries] bf16
 // Query rows of a step that go through the staging tile and the bulk reduction; the others are added from registers.
-// The first way is limited by shared memory (a write and a read of every float), the second by the load/store path;
-// each alone takes 870 us for a block of 4 096 x 4 096 with 32 heads, shared between them: 16 rows staged 843,
-// 24 842, 32 837, 36 826, 40 828, 44 828, 48 843.
+// The first way costs a shared-memory write and read of every float and two barriers, the second an instruction per
+// row and lane; each alone takes 870 us for a block of 4 096 x 4 096 with 32 heads, shared between them: 16 rows
+// staged 843, 24 842, 32 837, 36 826, 40 828, 44 828, 48 843.
 constexpr int kDqStaged = 40;
 constexpr int kDqStageBytes = kDqStaged * kBD * 4;
 constexpr int kFusedSmemBytes =
