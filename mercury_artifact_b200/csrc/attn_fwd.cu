@@ -35,6 +35,10 @@
 // arrival flag for its queries (they may still be in flight from another GPU) and a completion flag,
 // which the job's last CTA raises with a release store at system scope once every row of the job has
 // been stored -- the rows, and the flag, may live in another GPU's memory.
+//
+// A single job without flags may be cut differently (see plan_pack and plan_split): a tile then holds the rows of
+// all heads of a group, and an item's K/V tiles are shared between several CTAs, whose states
+// fwd_split_merge_kernel merges.
 #include <climits>
 
 #include "attn_fwd_common.cuh"
