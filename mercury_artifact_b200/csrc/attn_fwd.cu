@@ -1001,11 +1001,11 @@ static int launch_fwd(const mb_attn_fwd_multi_args* x, int pack_shift, const Fwd
     x_total = split.split_begin + split.slots;
   }
   dim3 grid(x_total, 1, 1);
-  // Short launches overlap their neighbours in the stream; what that saves per launch (100 queries against 16 384 keys,
-  // with the merge: 41.1 -> 38.8 us; 256 x 256, 8 heads: 17.0 -> 16.3 us) longer ones lose in the prologue of their later
-  // waves (384 items: 88.0 -> 89.0 us).  Launches with flags or several jobs stay in order: what they wait for may
+  // Launches of one wave overlap their neighbours in the stream; what that saves per launch (100 queries against 16 384
+  // keys, with the merge: 41.1 -> 38.8 us; 256 x 256, 8 heads: 17.0 -> 16.3 us) longer ones lose in the prologue of their
+  // later waves (384 items: 88.0 -> 89.0 us; 256 items: between 1 % faster and 1.6 % slower).  Launches with flags or several jobs stay in order: what they wait for may
   // need room on the SMs.
-  a.overlap = !has_flags && njobs == 1 && a.job[0].done_flag == nullptr && x_total <= 2 * sm_count();
+  a.overlap = !has_flags && njobs == 1 && a.job[0].done_flag == nullptr && x_total <= sm_count();
   if (a.overlap) {
     if (!launch_overlapped("launch attn_fwd_kernel", attn_fwd_kernel, grid, kFwdThreads, kFwdSmemBytes, stream, maps, a))
       return MB_E_CUDA;
