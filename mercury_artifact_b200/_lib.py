@@ -8,6 +8,7 @@ from __future__ import annotations
 
 import collections
 import ctypes as C
+import threading
 from pathlib import Path
 
 MB_MAX_SEGMENTS = 32
@@ -415,7 +416,10 @@ class StatusMonitor:
     post(stream) enqueues a copy of the device status word into pinned host memory behind the work
     just queued; poll() looks at the copies that have completed and raises if one is non-zero.  Ops
     call poll() when they begin and post() when they have enqueued their work, so a timeout surfaces
-    as an exception at the latest at the next call that finds the copy complete, or at check()."""
+    as an exception at the latest at the next call that finds the copy complete, or at check().
+
+    One monitor serves every op of a context, from any thread: the copies in flight are looked at and added to
+    under a lock (asking an event and queueing a copy both let other threads run)."""
 
     def __init__(self):
         import torch
@@ -427,8 +431,9 @@ class StatusMonitor:
         self._slots = {}
         self._free = {}   # per device: pairs to use again
         self._bad = 0
+        self._lock = threading.Lock()
 
-    def _reap(self) -> None:
+    def _reap(self) -> None:   # with the lock held
         for (device, _), slots in self._slots.items():
             while slots and slots[0][1].query():
                 host, ev = slots.popleft()
@@ -438,21 +443,23 @@ class StatusMonitor:
 
     def post(self, stream) -> None:
         torch = self._torch
-        self._reap()
-        free = self._free.get(stream.device_index)
-        if free:
-            host, ev = free.pop()
-        else:
-            host, ev = torch.zeros(1, dtype=torch.int32).pin_memory(), torch.cuda.Event()
-        check(lib.mb_status_peek_async(C.c_void_p(host.data_ptr()), C.c_void_p(stream.cuda_stream)),
-              "mb_status_peek_async")
-        ev.record(stream)
-        self._slots.setdefault((stream.device_index, stream.cuda_stream), collections.deque()).append((host, ev))
+        with self._lock:
+            self._reap()
+            free = self._free.get(stream.device_index)
+            if free:
+                host, ev = free.pop()
+            else:
+                host, ev = torch.zeros(1, dtype=torch.int32).pin_memory(), torch.cuda.Event()
+            check(lib.mb_status_peek_async(C.c_void_p(host.data_ptr()), C.c_void_p(stream.cuda_stream)),
+                  "mb_status_peek_async")
+            ev.record(stream)
+            self._slots.setdefault((stream.device_index, stream.cuda_stream), collections.deque()).append((host, ev))
 
     def poll(self) -> None:
-        self._reap()
-        if self._bad:
+        with self._lock:
+            self._reap()
             bad, self._bad = self._bad, 0
+        if bad:
             status_fetch(self._torch.cuda.current_stream().cuda_stream)   # synchronise and clear the device word
             raise MercuryB200Error(
                 f"a device-side wait of an earlier call timed out: {STATUS_NAMES.get(bad, bad)} (code {bad}); "

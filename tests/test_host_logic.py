@@ -303,3 +303,109 @@ def test_ring_divide_validation_and_memory_model():
     assert RingAttention((2,), 1, 4096, 32, 32, 128, causal=True, ctx=Ctx(), balance_causal=False,
                          ring_divide=7 if 4096 % 7 == 0 else 4).ring_divide == 4
     assert RingAttention((1,), 1, 4096, 32, 32, 128).memory_bytes() == {"symmetric": 0, "staging": 0, "inbox": 0, "state": 0}
+
+
+class _FakeCopies:
+    """Stands in for the device side of StatusMonitor: events complete when told to, every hand-over can be held up."""
+
+    def __init__(self, monkeypatch):
+        from mercury_artifact_b200 import _lib
+
+        self.on_query, self.on_peek = lambda ev: None, lambda stream: None
+        self.complete = set()
+        outer = self
+
+        class Event:
+            def record(self, stream):
+                self.stream = stream.cuda_stream
+
+            def query(self):
+                outer.on_query(self)
+                return self.stream in outer.complete
+
+        class Lib:
+            def mb_status_peek_async(self, host, stream):
+                outer.on_peek(stream.value)
+                return 0
+
+        monkeypatch.setattr(_lib, "lib", Lib())
+        monkeypatch.setattr(torch.cuda, "Event", Event)
+        monkeypatch.setattr(torch.Tensor, "pin_memory", lambda self: self)
+        self.monitor = _lib.StatusMonitor()
+
+    @staticmethod
+    def stream(handle):
+        return type("S", (), {"device_index": 0, "cuda_stream": handle})()
+
+    def pending(self):
+        return sorted(key[1] for key, slots in self.monitor._slots.items() for _ in slots)
+
+
+def _in_thread(fn):
+    import threading
+
+    failed = []
+
+    def body():
+        try:
+            fn()
+        except Exception as e:   # noqa: BLE001
+            failed.append(e)
+
+    t = threading.Thread(target=body)
+    t.failed = failed
+    t.start()
+    return t
+
+
+def test_status_monitor_post_during_another_threads_poll(monkeypatch):
+    """A thread whose post() on a new stream is under way while another polls: neither raises, nothing is lost."""
+    import threading
+
+    fake = _FakeCopies(monkeypatch)
+    fake.monitor.post(fake.stream(1))
+    at_peek, polled = threading.Event(), threading.Event()
+
+    def on_peek(handle):
+        if handle == 2:
+            at_peek.set()
+            polled.wait(0.5)
+
+    fake.on_peek = on_peek
+    poster = _in_thread(lambda: fake.monitor.post(fake.stream(2)))
+    assert at_peek.wait(5)
+
+    def on_query(ev):
+        polled.set()
+        poster.join(0.5)
+
+    fake.on_query = on_query
+    fake.monitor.poll()
+    poster.join(5)
+    assert not poster.is_alive() and not poster.failed
+    assert fake.pending() == [1, 2]
+
+
+def test_status_monitor_two_threads_take_one_completed_copy(monkeypatch):
+    """Two threads that look at the same completed copy: one takes it, the copy behind it stays pending (its pinned
+    word and its event are not handed out again while it is in flight)."""
+    fake = _FakeCopies(monkeypatch)
+    fake.monitor.post(fake.stream(1))
+    fake.monitor.post(fake.stream(1))
+    first = fake.monitor._slots[0, 1][0][1]
+    first.stream = "done"
+    fake.complete.add("done")
+    others = []
+
+    def on_query(ev):
+        if not others:
+            others.append(None)
+            others[0] = _in_thread(fake.monitor.poll)
+            others[0].join(0.3)
+
+    fake.on_query = on_query
+    fake.monitor.poll()
+    others[0].join(5)
+    assert not others[0].is_alive() and not others[0].failed
+    assert fake.pending() == [1]
+    assert [ev for pairs in fake.monitor._free.values() for _, ev in pairs] == [first]
