@@ -409,3 +409,22 @@ def test_status_monitor_two_threads_take_one_completed_copy(monkeypatch):
     assert not others[0].is_alive() and not others[0].failed
     assert fake.pending() == [1]
     assert [ev for pairs in fake.monitor._free.values() for _, ev in pairs] == [first]
+
+
+def test_stream_and_device_lookup_without_torch_private_functions(monkeypatch):
+    """The wrappers ask torch's C functions for the current device and stream (they are on every call's path), and the
+    documented ones where a torch does not have them."""
+    import importlib.util
+
+    from mercury_artifact_b200 import attention
+
+    monkeypatch.delattr(torch._C, "_cuda_getDevice")
+    monkeypatch.delattr(torch._C, "_cuda_getCurrentRawStream")
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 3)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda device: type("S", (), {"cuda_stream": 1000 + device})())
+    spec = importlib.util.spec_from_file_location("mercury_artifact_b200._attention_copy", attention.__file__)
+    copy = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(copy)
+    assert copy._stream_ptr() == 1003
+    assert copy._on(torch.device("cuda", 3)) is copy._SAME_DEVICE
+    assert isinstance(copy._on(torch.device("cuda", 1)), torch.cuda.device)
