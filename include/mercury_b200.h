@@ -83,7 +83,12 @@ MB_API int mb_attn_fwd(const mb_attn_fwd_args* args, void* cuda_stream);
  * filled last wave) are then split over their keys: the shares' rows, maxima and sums go through the
  * workspace in fp32 and a second kernel merges them.  mb_attn_fwd_workspace returns the bytes that the call
  * can use on the current device (0: none).  The workspace (16-byte aligned, contents arbitrary) belongs to
- * the call until its work on the stream is done; a smaller one, or NULL, runs the call unsplit. */
+ * the call until its work on the stream is done; a smaller one, or NULL, runs the call unsplit.
+ * Bits: a share takes its own reference maximum, so that its bf16 probabilities round at other places than
+ * those of an unsplit item.  The same call repeats bit for bit, but a row's bits may differ between launches of
+ * different shape (rows, heads, batch, keys, shards).  mb_attn_fwd, mb_attn_fwd_ws without a workspace and
+ * mb_attn_fwd_multi never split: one job over all shards, a chain of jobs over the same shards in the
+ * same order (see mb_fwd_job.state_*) and mb_attn_fwd agree bit for bit at every size. */
 MB_API int64_t mb_attn_fwd_workspace(const mb_attn_fwd_args* args);
 MB_API int mb_attn_fwd_ws(const mb_attn_fwd_args* args, void* workspace, uint64_t workspace_bytes, void* cuda_stream);
 

@@ -65,6 +65,9 @@ def attn_fwd_segments(
     given, is the address of a device int32 that reaches flag_value once the shard has
     arrived (the kernel waits for it before reading the shard).  Returns
     (o bf16 [b, sq, hq, d], lse fp32 [b, hq, sq]).
+
+    Items may be split over their keys (mb_attn_fwd_ws): a row's bits may then differ from those of
+    attn_fwd_multi, which never splits, and between calls of different shape.
     """
     _check_bshd(q, "q")
     b, sq, hq, d = q.shape

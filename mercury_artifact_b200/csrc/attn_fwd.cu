@@ -732,12 +732,6 @@ static int sm_count() {
   return count[dev];
 }
 
-// Without a split a launch of few items runs on as many SMs as it has items, and a last wave of few items leaves the
-// others idle.  Measured (B200), whole / split: 128 queries against 2 048 keys, 8 heads, 27 / 17 us; against 32 768 keys,
-// 315 / 41 us; 1 024 causal rows, 8 heads, 21 / 19 us; 4 096 queries against 32 768 keys, 32 heads (3.46 waves),
-// 1.92 / 1.80 ms with the last 68 items in 2 shares; 5 000 x 5 000, 16 heads, 234 / 188 us.  Shapes that the
-// costs below leave whole, and what a split did to them: 768 x 768, 8 heads, in 6 shares 19 -> 21 us; 2 048 x 4 096, 32
-// heads (108 items in the last wave), in 4 shares 132 -> 145 us.
 // log2 of the query heads that share a tile row by row (row = query * heads + head).  The heads of a group read the
 // same K/V, so a tile of 128 rows may hold all of them for 128 / group queries instead of one of them for 128:
 // worth it when the queries of one head leave much of a pair of tiles empty, which is where it saves an eighth of the
@@ -754,6 +748,12 @@ static int plan_pack(int sq, int hq, int hkv) {
   return packed * 8 <= apart * 7 ? shift : 0;
 }
 
+// Without a split a launch of few items runs on as many SMs as it has items, and a last wave of few items leaves the
+// others idle.  Measured (B200), whole / split: 128 queries against 2 048 keys, 8 heads, 27 / 17 us; against 32 768 keys,
+// 315 / 41 us; 1 024 causal rows, 8 heads, 21 / 19 us; 4 096 queries against 32 768 keys, 32 heads (3.46 waves),
+// 1.92 / 1.80 ms with the last 68 items in 2 shares; 5 000 x 5 000, 16 heads, 234 / 188 us.  Shapes that the
+// costs below leave whole, and what a split did to them: 768 x 768, 8 heads, in 6 shares 19 -> 21 us; 2 048 x 4 096, 32
+// heads (108 items in the last wave), in 4 shares 132 -> 145 us.
 static FwdSplit plan_split(const mb_attn_fwd_args* x) {
   const FwdSplit whole{INT_MAX, 1, 0};
   if (x->sq <= 0 || x->softmax_scale <= 0.f) return whole;
@@ -762,8 +762,11 @@ static FwdSplit plan_split(const mb_attn_fwd_args* x) {
   const int np = ((x->sq << pack_shift) + 2 * kBM - 1) / (2 * kBM), heads = x->hq >> pack_shift;
   const long long items = (long long)np * heads * x->batch;
   if (sms <= 0 || items > INT_MAX) return whole;
-  // A launch over several shards is cut in its last wave only: smaller ones add up in the order of the chained
-  // jobs of mb_attn_fwd_multi, whose results they equal bit for bit.
+  // Several shards: only the last wave of a non-causal launch is split.  Smaller launches and causal ones stay whole for
+  // callers that compare them with chained jobs (mb_attn_fwd_multi) bit for bit; what that costs, measured
+  // against one segment with the same keys: 256 queries, 8 heads, 8 shards of 256 keys 51 / 24 us, of 4 096
+  // keys 381 / 46 us; 1 024 causal rows, 8 shards of 1 024 keys 68 / 29 us.  From one wave up the equality
+  // holds for the whole items only.
   if (x->nseg > 1 && (x->causal || items < sms)) return whole;
   for (int s = 0; s < x->nseg; ++s)
     if (x->seg[s].ready_flag != nullptr) return whole;

@@ -469,3 +469,57 @@ def test_split_calls_and_merges_under_graph_capture():
         ro, rl = step()
         assert torch.equal(out, ro) and torch.equal(lse, rl)
     _status_ok()
+
+
+@pytest.mark.parametrize("B,Sq,H,hkv,causal,q_off,splits", [
+    (3, 6390, 2, 2, False, 0, True),     # 150 items, of which attn_fwd_segments splits the last two
+    (2, 300, 4, 2, True, 1100, False),   # heads of a group packed into a tile, which attn_fwd_multi does not do
+    (1, 100, 8, 2, True, 1300, False),
+])
+def test_ways_that_never_split_keep_each_others_bits(B, Sq, H, hkv, causal, q_off, splits):
+    """Over three shards, mb_attn_fwd (no workspace), one job of attn_fwd_multi and a chain of three jobs agree bit for
+    bit at every size, as mercury_b200.h says.  A call that splits agrees with them bit for bit in its whole
+    items and to the rounding of bf16 probabilities in the others."""
+    import mercury_artifact_b200 as mb
+    from mercury_artifact_b200.attention import attn_fwd_multi
+
+    Sk, D = 1400, 128
+    dev = torch.device("cuda", 0)
+    q, _, _, _ = seeded_qkv(11, B, Sq, H, hkv, D, device="cuda")
+    _, k, v, _ = seeded_qkv(12, B, Sk, H, hkv, D, device="cuda")
+    scale = D ** -0.5
+    cut = [Sk * i // 3 for i in range(4)]
+    segs = [(k[:, a:b], v[:, a:b], a) for a, b in zip(cut[:-1], cut[1:])]
+
+    def multi(masks):
+        o, lse = torch.empty_like(q), torch.empty(B, H, Sq, device=dev)
+        state = (torch.empty(B, H, Sq, D, device=dev), torch.empty(B, H, Sq, 2, device=dev))
+        chain = torch.zeros(B, H, (Sq + 255) // 256, dtype=torch.int32, device=dev)
+        jobs = [{"q": q, "q_off": q_off, "seg_mask": m} for m in masks]
+        for t, j in enumerate(jobs):
+            if len(jobs) > 1:
+                j.update(state=state, state_in=t > 0, state_out=t < len(jobs) - 1, chain=(chain.data_ptr(), t, t + 1))
+        jobs[-1]["out_raw"] = (o.data_ptr(), *o.stride()[:3])
+        jobs[-1]["lse_raw"] = (lse.data_ptr(), *lse.stride()[:2])
+        attn_fwd_multi(jobs, segs, scale, causal, B, H, hkv, D, dev)
+        return o, lse
+
+    o1, l1 = multi([7])
+    o3, l3 = multi([1, 2, 4])
+    ow, lw = torch.empty_like(q), torch.empty(B, H, Sq, device=dev)   # raw results: the wrapper gives no workspace
+    mb.attn_fwd_segments(q, segs, scale, causal=causal, q_off=q_off, out_raw=(ow.data_ptr(), *ow.stride()[:3]),
+                         lse_raw=(lw.data_ptr(), *lw.stride()[:2]))
+    os_, ls = mb.attn_fwd_segments(q, segs, scale, causal=causal, q_off=q_off)
+    _status_ok()
+    for o, lse in ((o3, l3), (ow, lw)):
+        assert torch.equal(o, o1) and torch.equal(lse, l1)
+    if not splits:
+        assert torch.equal(os_, o1) and torch.equal(ls, l1)
+        return
+    differ = (os_ != o1).any(-1)
+    whole = torch.ones_like(differ)
+    whole[2, 23 * 256:, 1] = False            # items 148 and 149: the last two pairs of tiles of the last head
+    assert not (differ & whole).any() and differ.any()
+    err = (os_.float() - o1.float())[~whole].norm() / o1.float()[~whole].norm()
+    assert err.item() <= 1e-2
+    assert (ls - l1).abs().max().item() <= LSE_TOL
