@@ -6,7 +6,7 @@ gradients on the same seeded inputs (Q/K/V/dO ~ N(0,1)*0.5).
 import pytest
 import torch
 
-from tests.helpers import golden_text, seeded_qkv, shard_inputs
+from tests.helpers import bwd_mass, golden_text, rounding_bound, seeded_qkv, shard_inputs
 
 pytestmark = pytest.mark.gpu
 
@@ -288,7 +288,9 @@ def test_row_statistics_and_zeroed_dq_buffer(Sq, shift):
 @pytest.mark.parametrize("Sq", [1, 39, 40, 41, 63, 64, 65, 104, 105, 127])
 def test_single_sweep_rows_of_the_last_step(Sq):
     """A step's 64 query rows reach the dQ buffer on two ways (40 through the staging tile, the others from registers):
-    every number of rows in the last step around both limits, and nothing past the last row."""
+    every number of rows in the last step around both limits, and nothing past the last row.  Every element keeps
+    the bound that the kernel's roundings give: dq is 0.01 in the mean of squares, and a key tile's contribution that is
+    lost in single rows moves it by less than G_TOL."""
     import mercury_artifact_b200 as mb
     from oracle import block
 
@@ -302,6 +304,8 @@ def test_single_sweep_rows_of_the_last_step(Sq):
     acc = torch.zeros(B, H, st.pad, D, device="cuda")
     dq, dk, dv = mb.attn_bwd_fused(q.cuda(), do.cuda(), st, k.cuda(), v.cuda(), scale, dq_accum=acc)
     _status_ok()
-    for got, want in ((dq, gq), (dk, gk), (dv, gv)):
-        assert (got.float().cpu() - want).abs().max().item() <= G_TOL
+    mass = bwd_mass(do, q, k, v, ro, rl, scale)
+    for got, want, m in ((dq, gq, mass[0]), (dk, gk, mass[1]), (dv, gv, mass[2]),
+                         (acc[:, :, :Sq].transpose(1, 2) * scale, gq, mass[0])):
+        assert ((got.float().cpu() - want).abs() <= rounding_bound(m, want)).all()
     assert (acc[:, :, Sq:] == 0).all()
