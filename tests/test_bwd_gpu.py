@@ -309,3 +309,113 @@ def test_single_sweep_rows_of_the_last_step(Sq):
                          (acc[:, :, :Sq].transpose(1, 2) * scale, gq, mass[0])):
         assert ((got.float().cpu() - want).abs() <= rounding_bound(m, want)).all()
     assert (acc[:, :, Sq:] == 0).all()
+
+
+def _spy(monkeypatch):
+    """Names of the library's functions in the order they are called."""
+    from mercury_artifact_b200 import _lib
+
+    called, real = [], _lib.lib
+
+    class Lib:
+        def __getattr__(self, name):
+            called.append(name)
+            return getattr(real, name)
+
+    monkeypatch.setattr(_lib, "lib", Lib())
+    return called
+
+
+BLOCK_CASES = [
+    # B, Sq, Sk, Hq, Hkv, causal
+    (2, 300, 300, 4, 4, False),
+    (1, 200, 450, 8, 2, True),     # bottom-right aligned, grouped heads
+    (1, 450, 200, 4, 2, True),     # the first 250 query rows see no key
+    (1, 1, 129, 4, 1, False),
+]
+
+
+@pytest.mark.parametrize("kind", ["one call", "packed dkv", "fp32 gradients", "out strides", "lse view", "mixed gradients"])
+@pytest.mark.parametrize("B,Sq,Sk,Hq,Hkv,causal", BLOCK_CASES)
+def test_block_backward_in_one_call_and_its_general_path(B, Sq, Sk, Hq, Hkv, causal, kind, monkeypatch):
+    """_flash_attn_backward hands tensors that share strides to mb_attn_bwd_block_sweep, others to the three functions it
+    consists of: both against the oracle, and dk / dv (no atomics) bit for bit against each other."""
+    import mercury_artifact_b200 as mb
+
+    q, _, _, do = seeded_qkv(61, B, Sq, Hq, Hq, 128)
+    _, k, v, _ = seeded_qkv(62, B, Sk, Hq, Hkv, 128)
+    scale = 128 ** -0.5
+    q_off = Sk - Sq if causal else 0
+    ro, rl, gq, gk, gv = _reference(q, k, v, do, scale, causal, q_off)
+    mass = bwd_mass(do, q, k, v, ro, rl, scale, causal, q_off)
+    qd, kd, vd, dod, ld = (x.cuda() for x in (q, k, v, do, rl))
+    od = torch.empty_like(qd).copy_(ro)
+    if kind == "out strides":
+        od = od.transpose(1, 2).contiguous().transpose(1, 2)
+        if od.stride() == qd.stride():
+            od = torch.cat([od, od], 3)[..., :128]
+    elif kind == "lse view":
+        ld = torch.stack([ld, ld], -1)[..., 0]
+    gq_type = torch.float32 if kind in ("fp32 gradients", "mixed gradients") else torch.bfloat16
+    gk_type = torch.float32 if kind == "fp32 gradients" else torch.bfloat16
+    dq = torch.full(qd.shape, float("nan"), dtype=gq_type, device="cuda")
+    if kind == "packed dkv":
+        dk, dv = torch.full((2, *kd.shape), float("nan"), dtype=gk_type, device="cuda")
+    else:
+        dk, dv = (torch.full(kd.shape, float("nan"), dtype=gk_type, device="cuda") for _ in range(2))
+    called = _spy(monkeypatch)
+    delta = mb._flash_attn_backward(dod, qd, kd, vd, od, ld, dq, dk, dv, 0.0, scale, causal)
+    monkeypatch.undo()
+    _status_ok()
+    one_call = kind in ("one call", "packed dkv", "fp32 gradients")
+    assert called == (["mb_attn_bwd_block_sweep"] if one_call else
+                      ["mb_attn_bwd_prepare_sweep", "mb_attn_bwd", "mb_attn_bwd_dq_convert"])
+    for got, want, m in ((dq, gq, mass[0]), (dk, gk, mass[1]), (dv, gv, mass[2])):
+        assert ((got.float().cpu() - want).abs() <= rounding_bound(m, want)).all()
+    prod = (do.double() * ro.double()).transpose(1, 2)
+    assert ((delta[:, :, :Sq].cpu() - prod.sum(-1)).abs() <= 128 * 2.0 ** -24 * prod.abs().sum(-1)).all()
+    st = mb.bwd_preprocess(dod, ro.cuda(), rl.cuda())
+    _, k2, v2 = mb.attn_bwd_fused(qd, dod, st, kd, vd, scale, causal=causal, q_off=q_off, dk=torch.empty_like(dk),
+                                  dv=torch.empty_like(dv), dq=torch.empty_like(dq))
+    assert torch.equal(dk, k2) and torch.equal(dv, v2) and torch.equal(delta, st.delta)
+
+
+@pytest.mark.parametrize("mode", ["dq", "dkv", "sweep"])
+def test_owner_tiles_in_uneven_head_blocks_keep_the_bits(mode):
+    """Causal launches take the owner tiles of several heads together, as many heads as have what they stream in 64 MiB:
+    more than one block of heads and a last one that is smaller (11 heads as 6 + 5, 11 as 4 + 4 + 3, 7 as 4 + 3).
+    A launch with an arrival flag (raised beforehand) goes head by head and gives the same bits."""
+    import mercury_artifact_b200 as mb
+    from mercury_artifact_b200.attention import _bwd_launch
+    from mercury_artifact_b200 import _lib
+
+    S, own, D = 16384, 300, 128
+    scale = D ** -0.5
+    hq, hkv = {"dq": (11, 11), "dkv": (22, 11), "sweep": (7, 7)}[mode]
+    sq, sk = (own, S) if mode == "dq" else (S, own)
+    q_off = S - own - 70 if mode == "dq" else -70      # rows without any key, tiles cut by the diagonal, whole ones
+    q, _, _, do = seeded_qkv(71, 1, sq, hq, hq, D, device="cuda")
+    _, k, v, _ = seeded_qkv(72, 1, sk, hq, hkv, D, device="cuda")
+    o, lse = mb.attn_fwd_segments(q, [(k, v, 0)], scale, causal=True, q_off=q_off)
+    st = mb.bwd_preprocess(do, o, lse)
+    flag = torch.ones(1, dtype=torch.int32, device="cuda")
+    results = []
+    for raised in ({}, {"flag": flag.data_ptr(), "flag_value": 1}):
+        if mode == "dq":
+            seg = {"str": k, "str_g": v, "off": 0, **raised}
+            results.append((mb.attn_bwd_dq(q, do, st, [seg], scale, causal=True, q_off=q_off),))
+            continue
+        seg = {"str": q, "str_g": do, "stats": st, "off": q_off, **raised}
+        dk, dv = torch.empty_like(k), torch.empty_like(v)
+        acc = torch.zeros(1, hq, st.pad, D, device="cuda") if mode == "sweep" else None
+        if mode == "sweep":
+            seg["dq_accum"] = acc
+        _bwd_launch(_lib.MB_BWD_MODE_FUSED if mode == "sweep" else _lib.MB_BWD_MODE_DKV, k, v, 0, [seg], hq, hkv, scale,
+                    True, dk, dv, False)
+        results.append((dk, dv, acc) if mode == "sweep" else (dk, dv))
+    _status_ok()
+    a, b = results
+    for x, y in zip(a[:2], b[:2]):
+        assert torch.equal(x, y) and x.float().abs().max().item() > 0
+    if mode == "sweep":   # three key tiles add to a row in any order
+        assert (a[2] - b[2]).abs().max().item() <= 2.0 ** -20 * a[2].abs().max().item()

@@ -539,3 +539,42 @@ def test_ways_that_never_split_keep_each_others_bits(B, Sq, H, hkv, causal, q_of
     err = (os_.float() - o1.float())[~whole].norm() / o1.float()[~whole].norm()
     assert err.item() <= 1e-2
     assert (ls - l1).abs().max().item() <= LSE_TOL
+
+
+@pytest.mark.parametrize("Sq,splits", [(600, True), (13900, False)])
+def test_items_in_uneven_head_blocks(Sq, splits, monkeypatch):
+    """Causal launches take the items of several heads together, as many heads as have their K/V in 64 MiB: 11 heads of
+    16 384 keys go as 6 + 5, with split items (and their merge) and without.  A launch with an arrival flag
+    (raised beforehand) goes head by head and whole, and gives the same bits where nothing was split."""
+    import mercury_artifact_b200 as mb
+    from mercury_artifact_b200 import _lib
+
+    Sk, H, D = 16384, 11, 128
+    scale = D ** -0.5
+    q_off = Sk - Sq - 50
+    q, _, _, _ = seeded_qkv(81, 1, Sq, H, H, D, device="cuda")
+    _, k, v, _ = seeded_qkv(82, 1, Sk, H, H, D, device="cuda")
+    real, need = _lib.lib, []
+
+    class Lib:
+        def __getattr__(self, name):
+            return getattr(real, name)
+
+        def mb_attn_fwd_workspace(self, args):
+            need.append(real.mb_attn_fwd_workspace(args))
+            return need[-1]
+
+    monkeypatch.setattr(_lib, "lib", Lib())
+    o, lse = mb.attn_fwd_segments(q, [(k, v, 0)], scale, causal=True, q_off=q_off)
+    monkeypatch.undo()
+    assert (need[0] > 0) == splits
+    flag = torch.ones(1, dtype=torch.int32, device="cuda")
+    seg = (k, v, 0, flag.data_ptr(), 1)
+    ow, lw = mb.attn_fwd_segments(q, [seg], scale, causal=True, q_off=q_off)
+    mass, _ = mb.attn_fwd_segments(q, [(k, v.abs(), *seg[2:])], scale, causal=True, q_off=q_off)
+    _status_ok()
+    if not splits:
+        assert torch.equal(o, ow) and torch.equal(lse, lw)
+    ow, mass = ow.float(), mass.float() * (1 + 2.0 ** -7)
+    assert ((o.float() - ow).abs() <= 2 * rounding_bound(mass, ow)).all()
+    assert (lse - lw).abs().max().item() <= 1e-5
