@@ -179,8 +179,8 @@ MB_API int mb_attn_bwd_prepare_sweep(const mb_bwd_preprocess_args* args, float* 
 
 #define MB_BWD_MODE_DKV 1 /* owner = one K/V shard, stream = query shards: writes dK (out1) and dV (out2) */
 #define MB_BWD_MODE_DQ 0  /* owner = one query shard, stream = K/V shards: writes dQ (out1) */
-#define MB_BWD_MODE_FUSED 2 /* like DKV, and each streamed query shard's dQ contributions are ADDED (fp32,
-                             * red.global.add) into its segment's dq_accum: scores are computed once, 5 tile
+#define MB_BWD_MODE_FUSED 2 /* like DKV, and each streamed query shard's dQ contributions are ADDED (fp32
+                             * reductions in L2) into its segment's dq_accum: scores are computed once, 5 tile
                              * products per block instead of 7.  dQ then depends on the order of fp32
                              * additions (not bitwise reproducible); finish with mb_attn_bwd_dq_convert. */
 #define MB_OUT_BF16 0

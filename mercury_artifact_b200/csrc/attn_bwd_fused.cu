@@ -13,9 +13,9 @@
 // [batch, hq, rows, head_dim] in global memory: the drain warps add 24 of the 64 query rows of a step with
 // red.global.add.f32 from registers (a lane holds one head-dim index, so a warp adds 128 contiguous bytes) and
 // transpose the other 40 through shared memory into rows of 128 floats (20 KiB, contiguous in the buffer)
-// that one thread adds with a bulk reduction (cp.reduce.async.bulk ... add.f32).  Without the additions the kernel
-// would take 751 us instead of 828 (4 096 x 4 096, 32 heads).  Each query row receives one contribution per K/V
-// tile that it can see.  A small kernel afterwards scales and converts the
+// that one thread adds with a bulk reduction (cp.reduce.async.bulk ... add.f32).  Block backward of 4 096 x 4 096,
+// 32 heads: 825 us, without the drain warps' work 703; with all rows on the second way 877, without its additions
+// 751.  Each query row receives one contribution per K/V tile that it can see.  A small kernel afterwards scales and converts the
 // buffer to bf16.  The order of those fp32 additions varies from run to run, so dQ is not
 // bitwise reproducible (dK and dV are); the two-launch form stays available for callers that
 // need determinism.
@@ -69,7 +69,11 @@ constexpr int kDsBytes = kOwnRows * kStrRows * 2;  // 16 KiB: dS^T as [128 keys]
 // Query rows of a step that go through the staging tile and the bulk reduction; the others are added from registers.
 // The first way costs a shared-memory write and read of every float and two barriers, the second an instruction per
 // row and lane; each alone takes 870 us for a block of 4 096 x 4 096 with 32 heads, shared between them: 16 rows
-// staged 843, 24 842, 32 837, 36 826, 40 828, 44 828, 48 843.
+// staged 843, 24 842, 32 837, 36 826, 40 828, 44 828, 48 843.  The values and the addresses of both ways live together:
+// 40 bytes of spill stores and 88 of loads with 128 launch registers (none when all rows were staged), 80 and 148 with
+// 120 (64 and 120).  The launches with flags, which take the latter, gain all the same (sweep alone, all rows staged /
+// two ways): 2 048 rows, 32/8 heads 223 / 212 us; 4 096 rows, 32/8 heads 884 / 837; 16 384 causal rows, 8/2
+// heads 1 749 / 1 682; 1 024 causal rows, 2 x 8 heads 37.2 / 35.1.
 constexpr int kDqStaged = 40;
 constexpr int kDqStageBytes = kDqStaged * kBD * 4;
 constexpr int kFusedSmemBytes =
@@ -341,7 +345,7 @@ __global__ void __maxnreg__(kLaunchRegs) attn_bwd_fused_kernel(const __grid_cons
     // idle: these two warps only complete the third warpgroup
     fused_regs_aux<kLaunchRegs>();
   } else if (warp >= 12) {
-    // ------------------------------------------------ drain dQ^T: tensor memory -> red.global.add
+    // ------------------------------------------------ drain dQ^T: tensor memory -> red.global.add and bulk reduction
     fused_regs_aux<kLaunchRegs>();
     const int quarter = warp & 3;
     const int d = (quarter << 5) | lane;  // head-dim index == tensor-memory lane
@@ -389,7 +393,8 @@ __global__ void __maxnreg__(kLaunchRegs) attn_bwd_fused_kernel(const __grid_cons
             float* dst = acc_base + (long long)(r0 + kDqStaged) * kBD + d;
             if (nrow >= kStrRows - kDqStaged) {
 #pragma unroll
-              for (int e = 0; e < kStrRows - kDqStaged; ++e) red_add(dst + e * kBD, v[(kDqStaged + e) >> 5][(kDqStaged + e) & 31]);
+              for (int e = 0; e < kStrRows - kDqStaged; ++e)
+                red_add(dst + e * kBD, v[(kDqStaged + e) >> 5][(kDqStaged + e) & 31]);
             } else {
 #pragma unroll
               for (int e = 0; e < kStrRows - kDqStaged; ++e)

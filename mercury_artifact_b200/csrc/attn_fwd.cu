@@ -671,7 +671,8 @@ struct FwdMergeArgs {
 // o = sum_p w_p O_p / sum_p w_p l_p with w_p = exp(scale * (m_p - max m)), in fp32.  A block handles 8 rows: warp w
 // columns [16 w, 16 w + 16), a lane 4 columns of one row, so that the lanes of a column group read 128 contiguous
 // bytes of a share and a row's 16 bf16 results are one 32-byte sector.  Latency-bound (the shares are in L2), hence
-// many small blocks and few registers, and a launch that overlaps the end of the attention kernel.
+// many small blocks and few registers.  After an attention launch of one wave its blocks are set up under the end of that
+// kernel; a longer one does not trigger it early (see launch_fwd) and is drained first.
 constexpr int kMergeRows = 8;
 __global__ void __launch_bounds__(256) fwd_split_merge_kernel(const FwdMergeArgs a) {
   constexpr int kRows = 2 * kBM;
@@ -887,7 +888,7 @@ static int launch_fwd(const mb_attn_fwd_multi_args* x, int pack_shift, const Fwd
     attr_set[dev] = true;
   }
 
-  // Kernel parameters (8.7 KB of tensor maps + 1.3 KB of scalars) are assembled in static storage:
+  // Kernel parameters (10.2 KB of tensor maps + 7.5 KB of jobs and scalars) are assembled in static storage:
   // the launch copies them, and launches of one process are issued from one thread at a time per device.
   static thread_local FwdMaps maps;
   static thread_local FwdArgs a;
@@ -1004,10 +1005,10 @@ static int launch_fwd(const mb_attn_fwd_multi_args* x, int pack_shift, const Fwd
     x_total = split.split_begin + split.slots;
   }
   dim3 grid(x_total, 1, 1);
-  // Launches of one wave overlap their neighbours in the stream; what that saves per launch (100 queries against 16 384
-  // keys, with the merge: 41.1 -> 38.8 us; 256 x 256, 8 heads: 17.0 -> 16.3 us) longer ones lose in the prologue of their
-  // later waves (384 items: 88.0 -> 89.0 us; 256 items: between 1 % faster and 1.6 % slower).  Launches with flags or several jobs stay in order: what they wait for may
-  // need room on the SMs.
+  // Launches of one wave overlap their neighbours in the stream; what that saves per launch (100 queries against
+  // 16 384 keys, with the merge: 41.1 -> 38.8 us; 256 x 256, 8 heads: 17.0 -> 16.3 us) longer ones lose in the
+  // prologue of their later waves (384 items: 88.0 -> 89.0 us; 256 items: between 1 % faster and 1.6 % slower).
+  // Launches with flags or several jobs stay in order: what they wait for may need room on the SMs.
   a.overlap = !has_flags && njobs == 1 && a.job[0].done_flag == nullptr && x_total <= sm_count();
   if (a.overlap) {
     if (!launch_overlapped("launch attn_fwd_kernel", attn_fwd_kernel, grid, kFwdThreads, kFwdSmemBytes, stream, maps, a))
