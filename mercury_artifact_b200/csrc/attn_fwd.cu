@@ -53,17 +53,25 @@ struct TileIter {
 __device__ __forceinline__ int seg_tiles(const FwdSmem* ctl, int s) {
   return max(ctl->n_tiles[0][s], ctl->n_tiles[1][s]);
 }
+// First tile of a segment that this CTA has (kCut: the launch splits items or packs heads).
+template <bool kCut>
+__device__ __forceinline__ int seg_first(const FwdSmem* ctl, int s) {
+  if constexpr (kCut) return ctl->t_lo[s];
+  return 0;
+}
+template <bool kCut>
 __device__ __forceinline__ TileIter iter_first(const FwdSmem* ctl, int nseg) {
   TileIter it{0, 0};
-  while (it.s < nseg && seg_tiles(ctl, it.s) <= ctl->t_lo[it.s]) ++it.s;
-  if (it.s < nseg) it.jt = ctl->t_lo[it.s];
+  while (it.s < nseg && seg_tiles(ctl, it.s) <= seg_first<kCut>(ctl, it.s)) ++it.s;
+  if (it.s < nseg) it.jt = seg_first<kCut>(ctl, it.s);
   return it;
 }
+template <bool kCut>
 __device__ __forceinline__ void iter_next(const FwdSmem* ctl, int nseg, TileIter& it) {
   if (++it.jt >= seg_tiles(ctl, it.s)) {
     ++it.s;
-    while (it.s < nseg && seg_tiles(ctl, it.s) <= ctl->t_lo[it.s]) ++it.s;
-    it.jt = it.s < nseg ? ctl->t_lo[it.s] : 0;
+    while (it.s < nseg && seg_tiles(ctl, it.s) <= seg_first<kCut>(ctl, it.s)) ++it.s;
+    it.jt = it.s < nseg ? seg_first<kCut>(ctl, it.s) : 0;
   }
 }
 
@@ -92,6 +100,11 @@ static_assert(8 * 32 * MB_FWD_SOFTMAX_REGS + 4 * 32 * MB_FWD_AUX_REGS <= kFwdThr
 
 // 160 registers/thread at launch (not the 168 that 384 threads would allow): the few warps' worth
 // left free on the SM let the transfer stream's one-thread flag kernels start beside a resident CTA.
+//
+// kCut: the launch splits items over their keys or packs the heads of a group.  The others, every launch with several jobs
+// among them, take an instantiation without what that needs, which short items feel (one instantiation / two): 8 x 256 x
+// 256, 32 heads 23.5 / 22.7 us, 16 x 256 x 256 49.3 / 47.7, 4 x 512 x 512 29.2 / 28.8; 8 192 x 8 192 the same.
+template <bool kCut>
 __global__ void __maxnreg__(MB_FWD_LAUNCH_REGS)
 attn_fwd_kernel(const __grid_constant__ FwdMaps maps, const __grid_constant__ FwdArgs a) {
   extern __shared__ uint8_t smem_raw[];
@@ -104,6 +117,7 @@ attn_fwd_kernel(const __grid_constant__ FwdMaps maps, const __grid_constant__ Fw
   const int tid = threadIdx.x;
   const int warp = tid >> 5;
   const int lane = tid & 31;
+  const int pack_shift = kCut ? a.pack_shift : 0;
 
   if (a.overlap) grid_dependents_launch();
   // Which job this CTA belongs to; within a job the heavier (later) query rows come first when causal.
@@ -115,16 +129,18 @@ attn_fwd_kernel(const __grid_constant__ FwdMaps maps, const __grid_constant__ Fw
     // CTAs are dispatched in grid order: job by job, inside a job in the order of item_coords (the CTAs
     // running at one time share a few heads' K/V through L2).
     int local = (int)blockIdx.x - a.job[jid].x_begin;
-    ctl->slot = -1;
-    ctl->part = 0;
-    if (local >= a.split_begin) {
-      ctl->slot = local - a.split_begin;
-      ctl->part = ctl->slot % a.nsplit;
-      local = a.split_begin + ctl->slot / a.nsplit;
+    if constexpr (kCut) {
+      ctl->slot = -1;
+      ctl->part = 0;
+      if (local >= a.split_begin) {
+        ctl->slot = local - a.split_begin;
+        ctl->part = ctl->slot % a.nsplit;
+        local = a.split_begin + ctl->slot / a.nsplit;
+      }
     }
-    const ItemCoords it = item_coords(local, a.job[jid].n_pairs, a.head_block, a.B, a.Hq >> a.pack_shift, a.causal);
+    const ItemCoords it = item_coords(local, a.job[jid].n_pairs, a.head_block, a.B, a.Hq >> pack_shift, a.causal);
     ctl->pair = it.pair;
-    ctl->h = it.h << a.pack_shift;
+    ctl->h = it.h << pack_shift;
     ctl->b = it.b;
   }
   __syncthreads();
@@ -159,10 +175,10 @@ attn_fwd_kernel(const __grid_constant__ FwdMaps maps, const __grid_constant__ Fw
     if (lane < a.nseg && ((J.seg_mask >> lane) & 1u)) {
 #pragma unroll
       for (int i = 0; i < 2; ++i)
-        n[i] = visible_tiles(q0 + i * kBM, J.Sq, a.pack_shift, J.q_off, a.causal, a.seg_sk[lane], a.seg_koff[lane]);
+        n[i] = visible_tiles(q0 + i * kBM, J.Sq, pack_shift, J.q_off, a.causal, a.seg_sk[lane], a.seg_koff[lane]);
     }
     int lo = 0;
-    if (ctl->slot >= 0) {
+    if (kCut && ctl->slot >= 0) {
       // This CTA's share of the item's walk over all its K/V tiles: an equal part, cut at whole tiles.
       const int mine = max(n[0], n[1]);
       int incl = mine;
@@ -179,7 +195,7 @@ attn_fwd_kernel(const __grid_constant__ FwdMaps maps, const __grid_constant__ Fw
       n[0] = min(n[0], hi);
       n[1] = min(n[1], hi);
     }
-    ctl->t_lo[lane] = lo;
+    if constexpr (kCut) ctl->t_lo[lane] = lo;
     ctl->n_tiles[0][lane] = n[0];
     ctl->n_tiles[1][lane] = n[1];
   }
@@ -196,7 +212,7 @@ attn_fwd_kernel(const __grid_constant__ FwdMaps maps, const __grid_constant__ Fw
   const uint32_t tmem = ctl->tmem_base;  // columns: S [0,128) P0 [128,192) P1 [192,256) O0 [256,384) O1 [384,512)
 
   bool any_work = false;
-  for (int s = 0; s < a.nseg; ++s) any_work |= seg_tiles(ctl, s) > ctl->t_lo[s];
+  for (int s = 0; s < a.nseg; ++s) any_work |= seg_tiles(ctl, s) > seg_first<kCut>(ctl, s);
 
   // Registers move from the auxiliary warpgroup (warps 8-11) to the two softmax
   // warpgroups; each role changes its own budget as the first thing it does.
@@ -216,12 +232,12 @@ attn_fwd_kernel(const __grid_constant__ FwdMaps maps, const __grid_constant__ Fw
         asm volatile("fence.proxy.async;" ::: "memory");
       }
       if (ok) {
-        const int rows = J.Sq << a.pack_shift;
+        const int rows = J.Sq << pack_shift;
         const int act0 = q0 < rows, act1 = q0 + kBM < rows;
         mbar_expect_tx(&ctl->q_full, (act0 + act1) * kTileBytes);
         for (int i = 0; i < 2; ++i) {
           if (q0 + i * kBM < rows) {
-            const int r0 = (q0 + i * kBM) >> a.pack_shift;
+            const int r0 = (q0 + i * kBM) >> pack_shift;
             tma_load_4d(sQ + i * kTileBytes, qmap, &ctl->q_full, 0, ctl->h, r0, ctl->b);
             tma_load_4d(sQ + i * kTileBytes + kHalfBytes, qmap, &ctl->q_full, 64, ctl->h, r0, ctl->b);
           }
@@ -231,7 +247,7 @@ attn_fwd_kernel(const __grid_constant__ FwdMaps maps, const __grid_constant__ Fw
       const int b_ = ctl->b, hkv = ctl->h / a.group;
       // One K or V tile into the next stage of the ring.
       auto load_tile = [&](int which, const TileIter& it) {
-        if (which == 0 && it.jt == ctl->t_lo[it.s] && a.seg_flag[it.s] != nullptr) {
+        if (which == 0 && it.jt == seg_first<kCut>(ctl, it.s) && a.seg_flag[it.s] != nullptr) {
           // The shard is being staged by another stream: wait (bounded) for its arrival flag,
           // then order the TMA reads (async proxy) after the flag read.
           ok = flag_wait_ge(a.seg_flag[it.s], a.seg_flag_value[it.s], abort_word, MB_ERR_TIMEOUT_SEGMENT,
@@ -252,17 +268,17 @@ attn_fwd_kernel(const __grid_constant__ FwdMaps maps, const __grid_constant__ Fw
         tma_load_4d(dst + kHalfBytes, map, &ctl->kv_full[stage], 64, hkv, it.jt * kBN, b_);
         ++n;
       };
-      TileIter nxt = iter_first(ctl, a.nseg);
+      TileIter nxt = iter_first<kCut>(ctl, a.nseg);
       TileIter cur = nxt;
       if (ok && nxt.s < a.nseg) {
         load_tile(0, nxt);
-        iter_next(ctl, a.nseg, nxt);
+        iter_next<kCut>(ctl, a.nseg, nxt);
       }
       while (ok && cur.s < a.nseg) {
         if (nxt.s < a.nseg) load_tile(0, nxt);
         if (ok) load_tile(1, cur);
         cur = nxt;
-        if (nxt.s < a.nseg) iter_next(ctl, a.nseg, nxt);
+        if (nxt.s < a.nseg) iter_next<kCut>(ctl, a.nseg, nxt);
       }
       if (!ok) {
         // Give copies already in flight a bounded chance to land before the CTA exits.
@@ -285,7 +301,7 @@ attn_fwd_kernel(const __grid_constant__ FwdMaps maps, const __grid_constant__ Fw
     if (any_work) {  // whole warp, converged
       constexpr uint32_t kStageUnits = kTileBytes / 16;
       int total = 0;  // K/V tiles this CTA walks through
-      for (int s = 0; s < a.nseg; ++s) total += max(seg_tiles(ctl, s) - ctl->t_lo[s], 0);
+      for (int s = 0; s < a.nseg; ++s) total += max(seg_tiles(ctl, s) - seg_first<kCut>(ctl, s), 0);
       bool ok = true;
       if (warp == 8) {
         constexpr uint32_t idesc_qk = umma_idesc_bf16(kBM, kBN, false, false);
@@ -297,7 +313,7 @@ attn_fwd_kernel(const __grid_constant__ FwdMaps maps, const __grid_constant__ Fw
         for (int s = 0; s < a.nseg && ok; ++s) {
           const int n0 = ctl->n_tiles[0][s], n1 = ctl->n_tiles[1][s];
           const int nmax = max(n0, n1);
-          for (int jt = ctl->t_lo[s]; jt < nmax && ok; ++jt, ++g) {
+          for (int jt = seg_first<kCut>(ctl, s); jt < nmax && ok; ++jt, ++g) {
             const int pos = g == 0 ? 0 : 2 * g - 1;
             const int stage = pos % kFwdStages;
             ok = mbar_wait_warp(&ctl->kv_full[stage], (pos / kFwdStages) & 1, abort_word, MB_ERR_TIMEOUT_KV_FULL, a.wait_cycles);
@@ -328,7 +344,7 @@ attn_fwd_kernel(const __grid_constant__ FwdMaps maps, const __grid_constant__ Fw
         for (int s = 0; s < a.nseg && ok; ++s) {
           const int n0 = ctl->n_tiles[0][s], n1 = ctl->n_tiles[1][s];
           const int nmax = max(n0, n1);
-          for (int jt = ctl->t_lo[s]; jt < nmax && ok; ++jt, ++g) {
+          for (int jt = seg_first<kCut>(ctl, s); jt < nmax && ok; ++jt, ++g) {
             const int pos = g == total - 1 ? 2 * total - 1 : 2 * g + 2;
             const int stage = pos % kFwdStages;
             ok = mbar_wait_warp(&ctl->kv_full[stage], (pos / kFwdStages) & 1, abort_word, MB_ERR_TIMEOUT_KV_FULL, a.wait_cycles);
@@ -379,8 +395,8 @@ attn_fwd_kernel(const __grid_constant__ FwdMaps maps, const __grid_constant__ Fw
     const uint32_t tOi = tmem + 256 + i * 128 + lane_field;
     // global position used by the causal rule (of the tile's first row: qfirst); the row inside the job's Q is
     // qpos - J.q_off
-    const int qfirst = J.q_off + ((q0 + i * kBM) >> a.pack_shift);
-    const int qpos = qfirst + (row >> a.pack_shift);
+    const int qfirst = J.q_off + ((q0 + i * kBM) >> pack_shift);
+    const int qpos = qfirst + (row >> pack_shift);
 
     float m_ref = -INFINITY;  // reference max (raw score units)
     float l = 0.f;            // running sum of exp2
@@ -427,7 +443,7 @@ attn_fwd_kernel(const __grid_constant__ FwdMaps maps, const __grid_constant__ Fw
       const int nt = ctl->n_tiles[i][s];
       const int sk = a.seg_sk[s];
       const int koff = a.seg_koff[s];
-      for (int jt = ctl->t_lo[s]; jt < nt; ++jt) {
+      for (int jt = seg_first<kCut>(ctl, s); jt < nt; ++jt) {
         ok = mbar_wait_warp(&ctl->s_full[i], cnt & 1, abort_word, MB_ERR_TIMEOUT_S, a.wait_cycles);
         if (!ok) break;
         tc_fence_after();
@@ -546,7 +562,7 @@ attn_fwd_kernel(const __grid_constant__ FwdMaps maps, const __grid_constant__ Fw
       if (ok) {
         const bool store = qrow < J.Sq;
         if (have_acc) tc_fence_after();
-        if (ctl->slot >= 0) {
+        if (kCut && ctl->slot >= 0) {
           // a share of the item: rows as they are, column group by column group (contiguous over a warp)
           const int r = i * kBM + row;
           if (cnt > 0) {
@@ -586,7 +602,7 @@ attn_fwd_kernel(const __grid_constant__ FwdMaps maps, const __grid_constant__ Fw
           if (store) *reinterpret_cast<float2*>(J.st_ml + st_row * 2) = make_float2(m_ref, l);
         } else {
           const float inv_l = (have_acc && l > 0.f) ? 1.f / l : 0.f;
-          const int head = ctl->h + (row & ((1 << a.pack_shift) - 1));
+          const int head = ctl->h + (row & ((1 << pack_shift) - 1));
           __nv_bfloat16* optr = J.o + (long long)ctl->b * J.o_sb + (long long)qrow * J.o_ss + (long long)head * J.o_sh;
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
@@ -882,8 +898,10 @@ static int launch_fwd(const mb_attn_fwd_multi_args* x, int pack_shift, const Fwd
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return MB_E_CUDA;
   if (dev < 64 && !attr_set[dev]) {
-    if (cudaFuncSetAttribute(attn_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFwdSmemBytes) !=
-        cudaSuccess)
+    if (cudaFuncSetAttribute(attn_fwd_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFwdSmemBytes) !=
+            cudaSuccess ||
+        cudaFuncSetAttribute(attn_fwd_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFwdSmemBytes) !=
+            cudaSuccess)
       return MB_E_CUDA;
     attr_set[dev] = true;
   }
@@ -1010,11 +1028,12 @@ static int launch_fwd(const mb_attn_fwd_multi_args* x, int pack_shift, const Fwd
   // prologue of their later waves (384 items: 88.0 -> 89.0 us; 256 items: between 1 % faster and 1.6 % slower).
   // Launches with flags or several jobs stay in order: what they wait for may need room on the SMs.
   a.overlap = !has_flags && njobs == 1 && a.job[0].done_flag == nullptr && x_total <= sm_count();
+  const auto kernel = split.slots > 0 || pack_shift > 0 ? attn_fwd_kernel<true> : attn_fwd_kernel<false>;
   if (a.overlap) {
-    if (!launch_overlapped("launch attn_fwd_kernel", attn_fwd_kernel, grid, kFwdThreads, kFwdSmemBytes, stream, maps, a))
+    if (!launch_overlapped("launch attn_fwd_kernel", kernel, grid, kFwdThreads, kFwdSmemBytes, stream, maps, a))
       return MB_E_CUDA;
   } else {
-    attn_fwd_kernel<<<grid, kFwdThreads, kFwdSmemBytes, stream>>>(maps, a);
+    kernel<<<grid, kFwdThreads, kFwdSmemBytes, stream>>>(maps, a);
     if (!cuda_ok(cudaGetLastError(), "launch attn_fwd_kernel")) return MB_E_CUDA;
   }
   if (split.slots > 0) {
