@@ -735,6 +735,7 @@ __global__ void __launch_bounds__(256) fwd_split_merge_kernel(const FwdMergeArgs
 struct FwdSplit {
   int split_begin, nsplit, slots;
 };
+constexpr FwdSplit kWhole{INT_MAX, 1, 0};
 constexpr size_t kSlotBytes = 2 * kBM * (kD * sizeof(float) + sizeof(float2));
 
 static int sm_count() {
@@ -765,17 +766,28 @@ static int plan_pack(int sq, int hq, int hkv) {
   return packed * 8 <= apart * 7 ? shift : 0;
 }
 
+// K/V tiles that a pair of query tiles walks through.
+static long long pair_tiles(const mb_attn_fwd_args* x, int pack_shift, int pair) {
+  const long long row = min(((pair + 1ll) * 2 * kBM - 1) >> pack_shift, x->sq - 1ll);  // the pair's last one
+  long long t = 0;
+  for (int s = 0; s < x->nseg; ++s) {
+    long long vis = x->seg[s].sk;
+    if (x->causal) vis = min(vis, x->q_off + row - x->seg[s].k_off + 1);
+    if (vis > 0) t += (vis + kBN - 1) / kBN;
+  }
+  return t;
+}
+
 // Without a split a launch of few items runs on as many SMs as it has items, and a last wave of few items leaves the
 // others idle.  Measured (B200), whole / split: 128 queries against 2 048 keys, 8 heads, 27 / 17 us; against 32 768 keys,
 // 315 / 41 us; 1 024 causal rows, 8 heads, 21 / 19 us; 4 096 queries against 32 768 keys, 32 heads (3.46 waves),
 // 1.92 / 1.80 ms with the last 68 items in 2 shares; 5 000 x 5 000, 16 heads, 234 / 188 us.  Shapes that the
 // costs below leave whole, and what a split did to them: 768 x 768, 8 heads, in 6 shares 19 -> 21 us; 2 048 x 4 096, 32
 // heads (108 items in the last wave), in 4 shares 132 -> 145 us.
-static FwdSplit plan_split(const mb_attn_fwd_args* x) {
-  const FwdSplit whole{INT_MAX, 1, 0};
+static FwdSplit plan_split(const mb_attn_fwd_args* x, int pack_shift) {
+  const FwdSplit whole = kWhole;
   if (x->sq <= 0 || x->softmax_scale <= 0.f) return whole;
   const int sms = sm_count();
-  const int pack_shift = plan_pack(x->sq, x->hq, x->hkv);
   const int np = ((x->sq << pack_shift) + 2 * kBM - 1) / (2 * kBM), heads = x->hq >> pack_shift;
   const long long items = (long long)np * heads * x->batch;
   if (sms <= 0 || items > INT_MAX) return whole;
@@ -789,18 +801,12 @@ static FwdSplit plan_split(const mb_attn_fwd_args* x) {
     if (x->seg[s].ready_flag != nullptr) return whole;
   // K/V tiles of the longest item, of the shortest one and of all items of a head
   long long t_max = 0, t_min = 0, t_sum = 0;
-  for (int s = 0; s < x->nseg; ++s) t_max += (max(x->seg[s].sk, 0) + kBN - 1) / kBN;
+  if (!x->causal) t_max = pair_tiles(x, pack_shift, 0);
   if (x->causal) {
     if (items > 4ll * sms) return whole;
-    t_min = t_max;
-    t_max = 0;
+    t_min = LLONG_MAX;
     for (int p = 0; p < np; ++p) {
-      long long t = 0;
-      const long long last = (long long)x->q_off + min(((p + 1) * 2 * kBM - 1) >> pack_shift, x->sq - 1);
-      for (int s = 0; s < x->nseg; ++s) {
-        const long long vis = min((long long)x->seg[s].sk, last - x->seg[s].k_off + 1);
-        if (vis > 0) t += (vis + kBN - 1) / kBN;
-      }
+      const long long t = pair_tiles(x, pack_shift, p);
       t_max = max(t_max, t);
       t_min = min(t_min, t);
       t_sum += t;
@@ -847,9 +853,40 @@ static FwdSplit plan_split(const mb_attn_fwd_args* x) {
   return best;
 }
 
+struct FwdPlan {
+  int pack_shift;
+  FwdSplit split;
+};
+
+// Heads are packed where plan_pack says so and the launch is split, or has more than one wave of pairs when the heads
+// stay apart.  Whole launches of one wave last as long as their longest pair, and a packed pair is a full one: only
+// where that pair has both tiles anyway and many steps does the smaller number of busy SMs (which clock higher)
+// make up for it.  Measured (B200), packed / apart: 4 x 128 x 128, 32 heads over 8, 9.2 / 7.4 us; 2 x 889 x 889
+// causal, 16 over 4, 18.9 / 17.1; 586 causal rows in 4 shards, 8 over 2, 31.0 / 29.3; 2 x 392 x 20 030 causal, 32
+// over 8, 248 / 255.  Non-causal launches of more waves need a fifth of the pairs saved (32 heads over 8: 4 x 440 x
+// 440, 256 -> 224 pairs, 30.3 / 28.9; 4 x 300 x 300, 256 -> 160, 24.7 / 26.7), causal ones, whose pairs are of many
+// lengths, do not (8 x 440 x 440, 512 -> 448, 43.2 / 46.7).
+static FwdPlan plan_fwd(const mb_attn_fwd_args* x, bool may_split) {
+  FwdPlan p{plan_pack(x->sq, x->hq, x->hkv), kWhole};
+  if (x->sq <= 0) return FwdPlan{0, kWhole};
+  if (may_split) p.split = plan_split(x, p.pack_shift);
+  if (p.pack_shift == 0 || p.split.slots > 0) return p;
+  const long long np = (x->sq + 2ll * kBM - 1) / (2 * kBM);
+  bool apart = false;
+  if (np * x->hq * x->batch <= sm_count()) {
+    const int rows = x->causal ? (x->sq - 1) % (2 * kBM) + 1 : min(x->sq, 2 * kBM);  // of the longest pair
+    apart = rows <= kBM || pair_tiles(x, 0, (int)np - 1) < 16;
+  } else if (!x->causal) {
+    const long long packed = (((long long)x->sq << p.pack_shift) + 2 * kBM - 1) / (2 * kBM);
+    apart = packed * 5 > (np << p.pack_shift) * 4;
+  }
+  if (apart) p = FwdPlan{0, may_split ? plan_split(x, 0) : kWhole};
+  return p;
+}
+
 long long attn_fwd_workspace(const mb_attn_fwd_args* x) {
   if (x == nullptr || x->nseg < 0 || x->nseg > MB_MAX_SEGMENTS || x->hq <= 0 || x->batch <= 0) return 0;
-  return plan_split(x).slots * (long long)kSlotBytes;
+  return plan_fwd(x, true).split.slots * (long long)kSlotBytes;
 }
 
 constexpr long long kL2Bytes = 64ll << 20;
@@ -1055,7 +1092,7 @@ static int launch_fwd(const mb_attn_fwd_multi_args* x, int pack_shift, const Fwd
 }
 
 int launch_attn_fwd_multi(const mb_attn_fwd_multi_args* x, cudaStream_t stream) {
-  return launch_fwd(x, 0, FwdSplit{INT_MAX, 1, 0}, nullptr, stream);
+  return launch_fwd(x, 0, kWhole, nullptr, stream);
 }
 
 // One query shard: the single-job form of the launch above.  With a workspace of attn_fwd_workspace(x) bytes the
@@ -1081,13 +1118,12 @@ int launch_attn_fwd(const mb_attn_fwd_args* x, void* ws, unsigned long long ws_b
   j.sq = x->sq; j.q_off = x->q_off;
   for (int s = 0; s < x->nseg; ++s) m.seg[s] = x->seg[s];
   m.status = x->status;
-  FwdSplit split{INT_MAX, 1, 0};
-  if (ws != nullptr && x->batch > 0 && x->hq > 0) {
-    split = plan_split(x);
-    if (split.slots * (unsigned long long)kSlotBytes > ws_bytes || (reinterpret_cast<uintptr_t>(ws) & 15u))
-      split = FwdSplit{INT_MAX, 1, 0};
+  FwdPlan plan{0, kWhole};
+  if (x->batch > 0 && x->hq > 0) {
+    plan = plan_fwd(x, ws != nullptr && (reinterpret_cast<uintptr_t>(ws) & 15u) == 0);
+    if (plan.split.slots * (unsigned long long)kSlotBytes > ws_bytes) plan = plan_fwd(x, false);
   }
-  return launch_fwd(&m, plan_pack(x->sq, x->hq, x->hkv), split, ws, stream);
+  return launch_fwd(&m, plan.pack_shift, plan.split, ws, stream);
 }
 
 }  // namespace mb

@@ -489,8 +489,10 @@ def test_split_calls_and_merges_under_graph_capture():
 
 @pytest.mark.parametrize("B,Sq,H,hkv,causal,q_off,splits", [
     (3, 6390, 2, 2, False, 0, True),     # 150 items, of which attn_fwd_segments splits the last two
-    (2, 300, 4, 2, True, 1100, False),   # heads of a group packed into a tile, which attn_fwd_multi does not do
+    (2, 300, 4, 2, True, 1100, False),   # one wave: whole, heads apart
     (1, 100, 8, 2, True, 1300, False),
+    (16, 300, 8, 2, True, 1100, False),  # 256 pairs with the heads of a group apart: packed (attn_fwd_multi does not)
+    (1, 180, 8, 2, True, 2500, False),   # one wave, both tiles of the longest pair and more than 16 key tiles: packed
 ])
 def test_ways_that_never_split_keep_each_others_bits(B, Sq, H, hkv, causal, q_off, splits):
     """Over three shards, mb_attn_fwd (no workspace), one job of attn_fwd_multi and a chain of three jobs agree bit for
@@ -499,7 +501,7 @@ def test_ways_that_never_split_keep_each_others_bits(B, Sq, H, hkv, causal, q_of
     import mercury_artifact_b200 as mb
     from mercury_artifact_b200.attention import attn_fwd_multi
 
-    Sk, D = 1400, 128
+    Sk, D = max(1400, Sq + q_off if causal else 0), 128
     dev = torch.device("cuda", 0)
     q, _, _, _ = seeded_qkv(11, B, Sq, H, hkv, D, device="cuda")
     _, k, v, _ = seeded_qkv(12, B, Sk, H, hkv, D, device="cuda")
