@@ -829,9 +829,14 @@ static FwdSplit plan_split(const mb_attn_fwd_args* x, int pack_shift) {
       if (items * ns <= sms) return longest;
       return max(longest, (total + items * ns * kCta) / sms + (double)t_min / ns + kCta);
     };
+    // Shares of more than one wave cost more than that: the merge waits for the launch to drain, and the shares of
+    // the third wave start late.  Measured less the sum above: 4 to 5 steps with 192 to 288 shares, 5 to 10 with
+    // 304 to 384.  8 heads, causal, whole / 2 shares: 4 352 rows 60.1 / 56.8 us, 4 864 (304 shares) 66.7 / 70.0,
+    // 5 000 68.8 / 74.3, 6 144 82.7 / 98.3; 4 heads, 9 728 rows 122.5 / 99.2.
+    auto late = [&](long long shares) { return shares > 2 * sms ? 7.5 : shares > sms ? 4.5 : 0.0; };
     double t_best = cost(1);
     for (int ns = 2; ns <= kMaxSplit && ns <= t_max && items * ns <= slot_cap; ++ns) {
-      const double t = cost(ns) + kMerge + kSlot * items * ns;
+      const double t = cost(ns) + kMerge + kSlot * items * ns + late(items * ns);
       if (t < t_best) {
         t_best = t;
         best = FwdSplit{0, ns, (int)(items * ns)};

@@ -580,3 +580,18 @@ def test_items_in_uneven_head_blocks(Sq, splits, monkeypatch):
     ow, mass = ow.float(), mass.float() * (1 + 2.0 ** -7)
     assert ((o.float() - ow).abs() <= 2 * rounding_bound(mass, ow)).all()
     assert (lse - lw).abs().max().item() <= 1e-5
+
+
+@pytest.mark.parametrize("rows,heads,splits", [(4352, 8, True), (4864, 8, False), (5000, 8, False), (6144, 8, False),
+                                               (2048, 8, True), (9728, 4, True)])
+def test_causal_launches_split_where_it_is_faster(rows, heads, splits):
+    """What mb_attn_fwd_workspace asks for around one wave of causal items (148 SMs): 4 864 to 6 144 rows with 8 heads were
+    split and slower for it, 9 728 rows with 4 heads have few long items; 2 048 rows take 2 shares, which fit a wave."""
+    from mercury_artifact_b200 import _lib
+
+    a = _lib.AttnFwdArgs()
+    a.batch, a.sq, a.hq, a.hkv, a.head_dim, a.causal, a.softmax_scale, a.nseg = 1, rows, heads, heads, 128, 1, 0.1, 1
+    a.seg[0].sk = rows
+    slots = _lib.lib.mb_attn_fwd_workspace(a) // (256 * (128 * 4 + 8))
+    items = (rows + 255) // 256 * heads
+    assert slots == (items * 2 if splits else 0)
