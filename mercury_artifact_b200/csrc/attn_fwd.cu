@@ -927,6 +927,16 @@ void set_peer_wait_ms(unsigned ms) { g_peer_wait_ms = ms == 0 ? 1 : ms; }
 // 2e6 cycles per millisecond is at least the requested time.
 long long peer_wait_cycles() { return g_peer_wait_ms * 2000000LL; }
 
+// What a launch of one wave loses per K/V step of its CTAs (in steps) when it follows another under overlap, at `busy` of
+// the SMs.  The two SMs of a TPC are slower when both work (64 steps: 103 us with up to 80 CTAs, 131 with 148).  An
+// ordinary launch of few CTAs puts one on each TPC; under overlap they go where the launch before leaves SMs free,
+// which comes out in pairs once the two together have more CTAs than SMs.  Measured back to back, overlapped / not,
+// 128 steps: 48 CTAs 0.99, 64 1.01, 80 1.07, 92 1.06, 108 1.04, 124 1.01, 140 0.99; 20 steps: 72 CTAs 0.94, 80 1.02.
+static double overlap_loss(double busy) {
+  if (busy < 0.33 || busy > 0.95) return 0.0;
+  return busy <= 0.5 ? 0.02 : 0.2 * (0.95 - busy);
+}
+
 // pack_shift != 0: one job without carried state or chain (see plan_pack).
 static int launch_fwd(const mb_attn_fwd_multi_args* x, int pack_shift, const FwdSplit& split, void* ws,
                       cudaStream_t stream) {
@@ -1065,11 +1075,23 @@ static int launch_fwd(const mb_attn_fwd_multi_args* x, int pack_shift, const Fwd
     x_total = split.split_begin + split.slots;
   }
   dim3 grid(x_total, 1, 1);
-  // Launches of one wave overlap their neighbours in the stream; what that saves per launch (100 queries against
-  // 16 384 keys, with the merge: 41.1 -> 38.8 us; 256 x 256, 8 heads: 17.0 -> 16.3 us) longer ones lose in the
+  // Launches of one wave overlap their neighbours in the stream, which saves about one K/V step (1.7 us; 100 queries
+  // against 16 384 keys, with the merge: 41.1 -> 38.8 us; 256 x 256, 8 heads: 17.0 -> 16.3 us), unless they lose more by
+  // it (see overlap_loss: 100 pairs of 50 steps, 83.6 without, 85.2 us with it).  Longer ones lose it in the
   // prologue of their later waves (384 items: 88.0 -> 89.0 us; 256 items: between 1 % faster and 1.6 % slower).
   // Launches with flags or several jobs stay in order: what they wait for may need room on the SMs.
-  a.overlap = !has_flags && njobs == 1 && a.job[0].done_flag == nullptr && x_total <= sm_count();
+  const int sms = sm_count();
+  a.overlap = !has_flags && njobs == 1 && a.job[0].done_flag == nullptr && x_total <= sms;
+  if (a.overlap) {
+    const FwdJob& J = a.job[0];
+    long long steps = 0;   // of the longest item
+    for (int s = 0; s < nseg; ++s) {
+      long long vis = (J.seg_mask >> s) & 1u ? a.seg_sk[s] : 0;
+      if (a.causal) vis = min(vis, (long long)J.q_off + J.Sq - a.seg_koff[s]);
+      if (vis > 0) steps += (vis + kBN - 1) / kBN;
+    }
+    a.overlap = (steps + split.nsplit - 1) / split.nsplit * overlap_loss((double)x_total / sms) <= 1.0;
+  }
   const auto kernel = split.slots > 0 || pack_shift > 0 ? attn_fwd_kernel<true> : attn_fwd_kernel<false>;
   if (a.overlap) {
     if (!launch_overlapped("launch attn_fwd_kernel", kernel, grid, kFwdThreads, kFwdSmemBytes, stream, maps, a))

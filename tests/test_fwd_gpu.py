@@ -595,3 +595,28 @@ def test_causal_launches_split_where_it_is_faster(rows, heads, splits):
     slots = _lib.lib.mb_attn_fwd_workspace(a) // (256 * (128 * 4 + 8))
     items = (rows + 255) // 256 * heads
     assert slots == (items * 2 if splits else 0)
+
+
+
+@pytest.mark.parametrize("heads,rows,keys", [(4, 5120, 1024), (4, 5120, 4096), (4, 2304, 4096), (4, 8960, 4096)])
+def test_launches_that_overlap_and_that_do_not_read_what_the_one_before_wrote(heads, rows, keys):
+    """Calls of one wave back to back, on both sides of the rule for overlapped launches (80 pairs of 8 and of 32 steps, 36
+    and 140 of 32), each on the output of the one before: the bits of the same calls with the device idle in between."""
+    import mercury_artifact_b200 as mb
+
+    q, _, _, _ = seeded_qkv(91, 1, rows, heads, heads, 128, device="cuda")
+    _, k, v, _ = seeded_qkv(92, 1, keys, heads, heads, 128, device="cuda")
+    half = keys // 2
+    segs = [(k[:, :half], v[:, :half], 0), (k[:, half:], v[:, half:], half)]
+
+    def chain(pause):
+        x = q
+        for _ in range(5):
+            x, lse = mb.attn_fwd_segments(x * 30.0, segs, 128 ** -0.5)
+            if pause:
+                torch.cuda.synchronize()
+        return x, lse
+
+    a, b = chain(False), chain(True)
+    _status_ok()
+    assert torch.equal(a[0], b[0]) and torch.equal(a[1], b[1])
