@@ -48,7 +48,7 @@ __global__ void __maxnreg__(160) attn_bwd_kernel(const __grid_constant__ BwdMaps
   volatile int* abort_word = &ctl->abort_word;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const OwnCoords own = own_coords(a, blockIdx.x);
+  const OwnCoords own = own_coords(a);
   const int own0 = own.tile * kOwnRows;
   const int h_own = own.h;  // dKV: kv head; dQ: query head
   const int b = own.b;
@@ -533,8 +533,8 @@ int launch_attn_bwd(const mb_attn_bwd_args* x, cudaStream_t stream) {
   a.n_heads = h_own;
   const long long heads = (long long)h_own * x->batch, n_ctas = heads * a.n_own;
   if (n_ctas > INT_MAX) return MB_E_INVALID;
-  a.head_block = 1;
-  if (a.causal && !has_flags) {
+  dim3 grid(a.n_own, h_own, x->batch);
+  if (a.causal && !has_flags && n_ctas > sm_count()) {
     // Longest tiles first, over as many heads as keep what they stream in kBwdL2Bytes of L2: per stream row
     // two bf16 rows, and in the single sweep an fp32 row of dQ that is added to.  Measured (B200, two
     // launches, 6 001 rows, 32 heads over 8, forward included): 1 540 us head by head, 1 480 with 16 MiB,
@@ -547,9 +547,12 @@ int launch_attn_bwd(const mb_attn_bwd_args* x, cudaStream_t stream) {
     const long long blocks = (heads + fit - 1) / fit;
     a.head_block = (int)((heads + blocks - 1) / blocks);
     a.own_last_first = dkv ? 0 : 1;
+  } else if (h_own > 65535 || x->batch > 65535) {
+    a.head_block = 1;
   }
-  if (fused) return launch_attn_bwd_fused(maps, a, (int)n_ctas, stream);
-  attn_bwd_kernel<0><<<(int)n_ctas, kBwdThreads, kBwdSmemBytes, stream>>>(maps, a);
+  if (a.head_block > 0) grid = dim3((unsigned)n_ctas);
+  if (fused) return launch_attn_bwd_fused(maps, a, grid, stream);
+  attn_bwd_kernel<0><<<grid, kBwdThreads, kBwdSmemBytes, stream>>>(maps, a);
   return cuda_ok(cudaGetLastError(), "launch attn_bwd_kernel") ? MB_SUCCESS : MB_E_CUDA;
 }
 

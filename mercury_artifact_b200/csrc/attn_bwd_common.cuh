@@ -51,17 +51,20 @@ struct BwdArgs {
   long long o_sb, o_ss, o_sh;
   int out_mode;  // 0 bf16 store, 1 fp32 store, 2 fp32 accumulate
   int* status;
-  // order of the owner tiles in the (one-dimensional) grid, see own_coords
+  // order of the owner tiles in the grid, see own_coords
   int n_own, n_heads, head_block, own_last_first;
 };
 
 // Owner tile, head and batch entry of a CTA.  (batch entry, head) pairs are taken in blocks of head_block; inside a
 // block the tiles come one after the other, the ones with the most steps first when causal, and the heads of
-// one tile position one after the other.  head_block = 1 is head by head.
+// one tile position one after the other.  head_block = 0: head by head in a three-dimensional grid, without the divisions
+// that delay a CTA's start (291 x 1 101, 32 heads, dQ: 22.0 us with them, 21.3 without).
 struct OwnCoords {
   int tile, h, b;
 };
-__device__ __forceinline__ OwnCoords own_coords(const BwdArgs& a, int item) {
+__device__ __forceinline__ OwnCoords own_coords(const BwdArgs& a) {
+  if (a.head_block == 0) return OwnCoords{(int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z};
+  const int item = blockIdx.x;
   const int blk = item / (a.head_block * a.n_own), rem = item - blk * a.head_block * a.n_own;
   const int n = min(a.head_block, a.B * a.n_heads - blk * a.head_block);  // heads of this block
   const int t = rem / n, bh = blk * a.head_block + rem % n;
@@ -237,6 +240,6 @@ __device__ __forceinline__ void ew_compute(const uint32_t (&xr)[32], const uint3
 }
 
 // single-pass kernel (attn_bwd_fused.cu), launched by launch_attn_bwd for MB_BWD_MODE_FUSED
-int launch_attn_bwd_fused(const BwdMaps& maps, const BwdArgs& a, int n_ctas, cudaStream_t stream);
+int launch_attn_bwd_fused(const BwdMaps& maps, const BwdArgs& a, dim3 grid, cudaStream_t stream);
 
 }  // namespace mb

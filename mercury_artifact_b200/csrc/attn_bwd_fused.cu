@@ -177,7 +177,7 @@ __global__ void __maxnreg__(kLaunchRegs) attn_bwd_fused_kernel(const __grid_cons
   }
   if (tid < MB_MAX_SEGMENTS) {  // one thread per segment: its range of 64-row steps for this owner tile
     int f = 0, l = 0;
-    const OwnCoords own = own_coords(a, blockIdx.x);
+    const OwnCoords own = own_coords(a);
     if (tid == 0) ctl->own = own;
     if (tid < a.nseg) step_range(a, own.tile * kOwnRows, tid, &f, &l);
     ctl->seg_first[tid] = f;
@@ -585,7 +585,7 @@ __global__ void __launch_bounds__(256) dq_convert_kernel(const DqConvertArgs a) 
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
-int launch_attn_bwd_fused(const BwdMaps& maps, const BwdArgs& a, int n_ctas, cudaStream_t stream) {
+int launch_attn_bwd_fused(const BwdMaps& maps, const BwdArgs& a, dim3 grid, cudaStream_t stream) {
   static bool done[64] = {};
   int dev = 0;
   if (!cuda_ok(cudaGetDevice(&dev), "cudaGetDevice")) return MB_E_CUDA;
@@ -602,8 +602,8 @@ int launch_attn_bwd_fused(const BwdMaps& maps, const BwdArgs& a, int n_ctas, cud
   // arrival flags are raised by one-warp kernels of the transfer stream: leave them room on every SM
   bool has_flags = false;
   for (int s = 0; s < a.nseg; ++s) has_flags |= a.seg_flag[s] != nullptr;
-  if (has_flags) attn_bwd_fused_kernel<120><<<n_ctas, kFusedThreads, kFusedSmemBytes, stream>>>(maps, a);
-  else attn_bwd_fused_kernel<128><<<n_ctas, kFusedThreads, kFusedSmemBytes, stream>>>(maps, a);
+  if (has_flags) attn_bwd_fused_kernel<120><<<grid, kFusedThreads, kFusedSmemBytes, stream>>>(maps, a);
+  else attn_bwd_fused_kernel<128><<<grid, kFusedThreads, kFusedSmemBytes, stream>>>(maps, a);
   return cuda_ok(cudaGetLastError(), "launch attn_bwd_fused_kernel") ? MB_SUCCESS : MB_E_CUDA;
 }
 

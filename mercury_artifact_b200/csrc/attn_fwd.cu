@@ -738,7 +738,7 @@ struct FwdSplit {
 constexpr FwdSplit kWhole{INT_MAX, 1, 0};
 constexpr size_t kSlotBytes = 2 * kBM * (kD * sizeof(float) + sizeof(float2));
 
-static int sm_count() {
+int sm_count() {
   static int count[64] = {};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;

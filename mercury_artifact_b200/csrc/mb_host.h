@@ -34,6 +34,9 @@ bool launch_overlapped(const char* what, void (*kernel)(Params...), dim3 grid, i
   return cuda_ok(cudaLaunchKernelEx(&cfg, kernel, args...), what);
 }
 
+// SMs of the current device (0 on failure).
+int sm_count();
+
 // Device address of the library's status word on the current device (nullptr on failure).
 int* default_status_word();
 
